@@ -54,7 +54,8 @@ struct obl_ctx {
     double *d_kx = nullptr;    // kx(lhx), Nyquist 0
     double *d_ky1 = nullptr;   // ky(lhy), Nyquist 0 (1D, for ddy)
     double *d_ky2 = nullptr;   // ky_2d row (nyt), Nyquist row 0
-    std::map<int, void *> tw;  // 4*n + role -> plan twiddle table in the storage precision
+    std::map<int, void *> tw;  // 8*n + role -> plan twiddle table in the storage precision (in d_tw)
+    void *d_tw = nullptr;
     // FP64 islands (mixed mode)
     int n_isl = 0;
     int *d_isl = nullptr;
@@ -189,7 +190,7 @@ static int ensure(obl_ctx *ctx, DevBuf &b, size_t bytes)
 
 template <typename T> static const C2<T> *twt(obl_ctx *c, int n, int role)
 {
-    return (const C2<T> *)c->tw.at(4 * n + role);
+    return (const C2<T> *)c->tw.at(8 * n + role);
 }
 
 static bool len_ok(int n) { return line_length_supported(n); }
@@ -215,12 +216,12 @@ template <typename T> struct Ops {
     }
 
     // plan twiddle tables of the forward / backward transform of a line op of base length n
-    void tables(int op, int n, const C2<T> *&f, const C2<T> *&b)
+    void tables(int op, int n, const C2<T> *&f, const C2<T> *&b, int family)
     {
         const int rf = op == OP_UNPAD ? ROLE_PADFWD : ROLE_FWD;
         const int rb = op == OP_PAD ? ROLE_PADBWD : ROLE_BWD;
-        f = twt<T>(ctx, n, rf);
-        b = twt<T>(ctx, n, rb);
+        f = twt<T>(ctx, n, family + rf);
+        b = twt<T>(ctx, n, family + rb);
     }
     RowArgs<T> rowargs(const void *src, long long ss, void *dst, long long ds, long long nrows, double scale,
                        int op, int n)
@@ -228,17 +229,17 @@ template <typename T> struct Ops {
         RowArgs<T> a{};
         a.src = src; a.dst = dst; a.src_stride = ss; a.dst_stride = ds; a.npairs = nrows / 2;
         a.scale = (T)scale; a.ktab = ctx->d_kx;
-        tables(op, n, a.twF, a.twB);
+        tables(op, n, a.twF, a.twB, ROLE_TP);
         a.pad_scale = (T)1; a.pad_mode = 0;
         return a;
     }
     ColArgs<T> colargs(const void *src, long long srow, long long spl, void *dst, long long drow, long long dpl,
-                       int ncols, int nlev, double scale, int op, int n)
+                       int ncols, int nlev, double scale, int op, int n, int family = ROLE_TP)
     {
         ColArgs<T> a{};
         a.src = src; a.dst = dst; a.src_row = srow; a.dst_row = drow; a.src_plane = spl; a.dst_plane = dpl;
         a.ncols = ncols; a.nlev = nlev; a.scale = (T)scale; a.ktab = ctx->d_ky1;
-        tables(op, n, a.twF, a.twB);
+        tables(op, n, a.twF, a.twB, family);
         a.pad_copy = 0; a.zero_nyq = 0; a.kmul = 0;
         return a;
     }
@@ -625,7 +626,7 @@ template <typename T> struct Ops {
             pc.ph = ph; pc.dph = (const C2<T> *)ctx->spec[4].p;
             pc.Xp = Hz; pc.Xdy = Hy; pc.Xdz = (C2<T> *)ctx->spec[4].p;
             pc.S = S; pc.lhx = lhx; pc.kx = ctx->d_kx; pc.ky = ctx->d_ky2;
-            pc.twB = twt<T>(ctx, ny, ROLE_BWD);
+            pc.twB = twt<T>(ctx, ny, ROLE_TP + ROLE_BWD);
             {
                 LaunchScope ls(ctx->rec, "pinv_cols", s());
                 if ((rc = chk(PinvLaunch<T>::cols(ny, pc, L + 1, s()), "pinv_cols"))) return rc;
@@ -637,7 +638,7 @@ template <typename T> struct Ops {
             pr.npairs = (long long)ny * (L + 1) / 2;
             pr.ldx = ldx; pr.ny = ny; pr.lhx = lhx;
             pr.dt_tadv1 = (T)(ctx->dt_nd * kTadv1);
-            pr.twB = twt<T>(ctx, nx, ROLE_BWD);
+            pr.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD);
             {
                 LaunchScope ls(ctx->rec, "pinv_rows_project", s());
                 if ((rc = chk(PinvLaunch<T>::rows(nx, pr, s()), "pinv_rows_project"))) return rc;
@@ -725,7 +726,7 @@ template <typename T> struct Ops {
         int rc = rows(OP_DERIV, ctx->nxt, ra, "divt_ddx_rows");
         if (rc) return rc;
         auto ca = colargs(ty + pl, ctx->ldx, pl, divt + pl, ctx->ldx, pl, ctx->nxt, nlev, 1.0 / ctx->nyt, OP_DERIV,
-                          ctx->nyt);
+                          ctx->nyt, 0);
         ca.ktab = ctx->d_ky1;
         DivEpi<T> ep{};
         ep.out = divt + pl;
@@ -829,8 +830,8 @@ template <typename T> struct Ops {
             ra.src = f[c] + pl * z0; ra.dfdx = (T *)io->d[2 * c] + pl * z0; ra.xpad = xb; ra.H = H ? H + S * z0 : nullptr;
             ra.npairs = (long long)ny * nl / 2; ra.ldx = ctx->ldx; ra.ny = ny; ra.L = ctx->L; ra.z0 = z0;
             ra.sc_press = scp; ra.kx = ctx->d_kx;
-            ra.twF = twt<T>(ctx, nx, ROLE_FWD); ra.twB = twt<T>(ctx, nx, ROLE_BWD);
-            ra.twPB = twt<T>(ctx, nx, ROLE_PADBWD);
+            ra.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD); ra.twB = twt<T>(ctx, nx, ROLE_TP + ROLE_BWD);
+            ra.twPB = twt<T>(ctx, nx, ROLE_TP + ROLE_PADBWD);
             {
                 LaunchScope ls(ctx->rec, "rows_fwd3", s());
                 if ((rc = chk(RowsFwd3Launch<T>::run(nx, ra, s()), "rows_fwd3"))) return rc;
@@ -1204,7 +1205,7 @@ template <typename T> struct Ops {
         C2<T> *ph = (C2<T> *)ctx->spec[3].p, *dph = (C2<T> *)ctx->spec[4].p;
         PinvColArgs<T> pc{};
         pc.ph = ph; pc.dph = dph; pc.Xp = Hz; pc.Xdy = Hy; pc.Xdz = dph;
-        pc.S = S; pc.lhx = lhx; pc.kx = ctx->d_kx; pc.ky = ctx->d_ky2; pc.twB = twt<T>(ctx, ny, ROLE_BWD);
+        pc.S = S; pc.lhx = lhx; pc.kx = ctx->d_kx; pc.ky = ctx->d_ky2; pc.twB = twt<T>(ctx, ny, ROLE_TP + ROLE_BWD);
         {
             LaunchScope ls(ctx->rec, "pinv_cols", s());
             if ((rc = chk(PinvLaunch<T>::cols(ny, pc, L + 1, s()), "pinv_cols"))) return rc;
@@ -1216,7 +1217,7 @@ template <typename T> struct Ops {
         pr.npairs = (long long)ny * (L + 1) / 2;
         pr.ldx = ldx; pr.ny = ny; pr.lhx = lhx;
         pr.dt_tadv1 = (T)(ctx->dt_nd * kTadv1);
-        pr.twB = twt<T>(ctx, nx, ROLE_BWD);
+        pr.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD);
         pr.w_from_1 = rank > 0;   // jz_min = 2 only on the bottom rank (110_project.f90:29-33)
         {
             LaunchScope ls(ctx->rec, "pinv_rows_project", s());
@@ -1251,7 +1252,7 @@ template <typename T> struct Ops {
         C2<T> *ph = (C2<T> *)ctx->spec[3].p, *dph = (C2<T> *)ctx->spec[4].p;
         const T *f[4] = {(const T *)io->u, (const T *)io->v, (const T *)io->w, (const T *)io->theta};
         const double scp = ((1.0 / ((double)nx * ny)) / kTadv1) * (1.0 / ctx->dt_nd);
-        const int WB = ens_wb<T>();
+        const int WB = ens_lines_of(ny);
         I = EnsInst<T>{};
         I.nx = nx; I.ny = ny; I.nlev = nlev; I.L = L;
         for (int c = 0; c < 4; ++c) {
@@ -1260,8 +1261,8 @@ template <typename T> struct Ops {
             ra.src = f[c]; ra.dfdx = (T *)io->d[2 * c]; ra.xpad = xb; ra.H = c < 3 ? H[c] : nullptr;
             ra.npairs = (long long)ny * nlev / 2; ra.ldx = ldx; ra.ny = ny; ra.L = L; ra.z0 = 0;
             ra.sc_press = scp; ra.kx = ctx->d_kx;
-            ra.twF = twt<T>(ctx, nx, ROLE_FWD); ra.twB = twt<T>(ctx, nx, ROLE_BWD);
-            ra.twPB = twt<T>(ctx, nx, ROLE_PADBWD);
+            ra.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD); ra.twB = twt<T>(ctx, nx, ROLE_TP + ROLE_BWD);
+            ra.twPB = twt<T>(ctx, nx, ROLE_TP + ROLE_PADBWD);
             I.padc[c] = colargs(xb, nx2, (long long)nx2 * ny, io->big[c], nx2, (long long)nx2 * ny2, nx2, nlev,
                                 1.0 / ny, OP_PAD, ny);
             I.ddyc[c] = colargs(f[c], ldx, ctx->plane(), io->d[2 * c + 1], ldx, ctx->plane(), nx, nlev, 1.0 / ny,
@@ -1289,8 +1290,8 @@ template <typename T> struct Ops {
         I.bulk_units = (S + 255) / 256;
         PinvColArgs<T> &pc = I.pc;
         pc.ph = ph; pc.dph = dph; pc.Xp = H[2]; pc.Xdy = H[1]; pc.Xdz = dph;
-        pc.S = S; pc.lhx = lhx; pc.kx = ctx->d_kx; pc.ky = ctx->d_ky2; pc.twB = twt<T>(ctx, ny, ROLE_BWD);
-        I.pc_nb = (lhx + WB - 1) / WB;
+        pc.S = S; pc.lhx = lhx; pc.kx = ctx->d_kx; pc.ky = ctx->d_ky2; pc.twB = twt<T>(ctx, ny, ROLE_TP + ROLE_BWD);
+        I.pc_nb = I.fwd_nb + (I.fwd_nb + 1) / 2;   // p_hat's line groups, and pairs of the dpdz spectrum's
         PinvRowArgs<T> &pr = I.pr;
         pr.Xp = H[2]; pr.kx = ctx->d_kx; pr.Xdy = H[1]; pr.Xdz = dph;
         pr.p = (T *)io->p; pr.dpdx = (T *)io->dp[0]; pr.dpdy = (T *)io->dp[1]; pr.dpdz = (T *)io->dp[2];
@@ -1298,7 +1299,7 @@ template <typename T> struct Ops {
         pr.npairs = (long long)ny * (L + 1) / 2;
         pr.ldx = ldx; pr.ny = ny; pr.lhx = lhx;
         pr.dt_tadv1 = (T)(ctx->dt_nd * kTadv1);
-        pr.twB = twt<T>(ctx, nx, ROLE_BWD);
+        pr.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD);
         I.pr_units = EnsGeoHost<T>::pinv_rows_units(nx, pr.npairs);
         I.u = (T *)io->u; I.v = (T *)io->v; I.w = (T *)io->w;
         I.ldx = ldx; I.nz = ctx->nz; I.stress_free = (int)ctx->opt.ubc_stress_free;
@@ -1490,26 +1491,29 @@ int obl_ctx_create(const obl_grid *grid, const obl_options *opt, obl_ctx **out)
     if (cudaMemset(ctx->d_ctl, 0, 4 * sizeof(int)) != cudaSuccess) return bad(OBL_ERR_CUDA);
 
     // plan twiddle tables (FP64 on the host, stored in the storage precision) for the
-    // forward / backward / padded transforms of both horizontal lengths
-    for (int n : {ctx->nxt, ctx->nyt})
-        for (int role = 0; role < 4; ++role) {
-            const int key = 4 * n + role;
-            if (ctx->tw.count(key)) continue;
-            const std::vector<double> h = plan_table(n, role);
-            const size_t m = h.size() / 2;
-            const size_t b = (ctx->f64 ? sizeof(double2) : sizeof(float2)) * (m > 0 ? m : 1);
-            void *d = nullptr;
-            if (dev_malloc(ctx, &d, b) != cudaSuccess) return bad(OBL_ERR_NOMEM);
-            ctx->tw[key] = d;
-            if (m == 0) continue;
-            if (ctx->f64) {
-                if (cudaMemcpy(d, h.data(), b, cudaMemcpyHostToDevice) != cudaSuccess) return bad(OBL_ERR_CUDA);
-            } else {
-                std::vector<float2> hf(m);
-                for (size_t i = 0; i < m; ++i) hf[i] = make_float2((float)h[2 * i], (float)h[2 * i + 1]);
-                if (cudaMemcpy(d, hf.data(), b, cudaMemcpyHostToDevice) != cudaSuccess) return bad(OBL_ERR_CUDA);
+    // forward / backward / padded transforms of both horizontal lengths, in one allocation
+    {
+        const size_t eb = ctx->f64 ? sizeof(double2) : sizeof(float2);
+        std::vector<unsigned char> all;
+        std::map<int, size_t> at;
+        for (int n : {ctx->nxt, ctx->nyt})
+            for (int role = 0; role < 2 * ROLE_TP; ++role) {
+                const int key = 8 * n + role;
+                if (at.count(key)) continue;
+                const std::vector<double> h = plan_table(n, role);
+                at[key] = all.size();
+                all.resize((all.size() + eb * (h.size() / 2) + 255) / 256 * 256);
+                unsigned char *p = all.data() + at[key];
+                if (ctx->f64) {
+                    if (!h.empty()) std::memcpy(p, h.data(), sizeof(double) * h.size());
+                } else {
+                    for (size_t i = 0; i < h.size(); ++i) reinterpret_cast<float *>(p)[i] = (float)h[i];
+                }
             }
-        }
+        if (dev_malloc(ctx, &ctx->d_tw, all.size() + 256) != cudaSuccess) return bad(OBL_ERR_NOMEM);
+        for (auto &kv : at) ctx->tw[kv.first] = (unsigned char *)ctx->d_tw + kv.second;
+        if (cudaMemcpy(ctx->d_tw, all.data(), all.size(), cudaMemcpyHostToDevice) != cudaSuccess) return bad(OBL_ERR_CUDA);
+    }
 
     // FP64 islands of the mixed mode: the (0,0) mean mode and every column with
     // k^2 <= fp64_k2_max (weakly diagonally dominant systems)
@@ -1559,7 +1563,7 @@ int obl_ctx_destroy(obl_ctx *ctx)
     cudaFree(ctx->d_ky2);
     cudaFree(ctx->d_isl);
     cudaFree(ctx->d_skip);
-    for (auto &kv : ctx->tw) cudaFree(kv.second);
+    cudaFree(ctx->d_tw);
     for (auto &b : ctx->spec) cudaFree(b.p);
     cudaFree(ctx->cscr.p);
     cudaFree(ctx->isl_c.p);
@@ -2566,10 +2570,10 @@ int ens_ctx_fail(obl_ensemble *ens, int i, int rc)
 // builds and uploads the work list of the persistent kernel for these buffers
 // the launches of the persistent step: phase ranges and CTAs per SM of each
 struct EnsPart {
-    int pb, pe, minb;
+    int pb, pe;
 };
-static const EnsPart kEnsAll[1] = {{0, 6, OBL_ENS_MINB}};
-static const EnsPart kEnsSplit[3] = {{0, 1, 2}, {1, 4, 4}, {4, 6, 2}};
+static const EnsPart kEnsAll[1] = {{0, 6}};
+static const EnsPart kEnsSplit[3] = {{0, 1}, {1, 4}, {4, 6}};
 
 static bool ens_persistent(int mode)
 {
@@ -2577,19 +2581,19 @@ static bool ens_persistent(int mode)
 }
 template <typename T> static int ens_part_bps(const EnsPart &p, size_t smem, bool flow)
 {
-    if (flow) return EnsFlowKernel<T, OBL_ENS_MINB>::blocks_per_sm(smem);
-    if (p.pb == 0 && p.pe == 6) return EnsKernel<T, 0, 6, OBL_ENS_MINB>::blocks_per_sm(smem);
+    if (flow) return EnsFlowKernel<T, ens_minb<T>()>::blocks_per_sm(smem);
+    if (p.pb == 0 && p.pe == 6) return EnsKernel<T, 0, 6, ens_minb<T>()>::blocks_per_sm(smem);
     if (p.pb == 0) return EnsKernel<T, 0, 1, 2>::blocks_per_sm(smem);
-    if (p.pb == 1) return EnsKernel<T, 1, 4, 4>::blocks_per_sm(smem);
+    if (p.pb == 1) return EnsKernel<T, 1, 4, ens_minb_mid<T>()>::blocks_per_sm(smem);
     return EnsKernel<T, 4, 6, 2>::blocks_per_sm(smem);
 }
 template <typename T> static cudaError_t ens_part_launch(const EnsPart &p, const EnsArgs<T> &a, int blocks, size_t smem,
                                                         cudaStream_t s, bool flow)
 {
-    if (flow) return EnsFlowKernel<T, OBL_ENS_MINB>::launch(a, blocks, smem, s);
-    if (p.pb == 0 && p.pe == 6) return EnsKernel<T, 0, 6, OBL_ENS_MINB>::launch(a, blocks, smem, s);
+    if (flow) return EnsFlowKernel<T, ens_minb<T>()>::launch(a, blocks, smem, s);
+    if (p.pb == 0 && p.pe == 6) return EnsKernel<T, 0, 6, ens_minb<T>()>::launch(a, blocks, smem, s);
     if (p.pb == 0) return EnsKernel<T, 0, 1, 2>::launch(a, blocks, smem, s);
-    if (p.pb == 1) return EnsKernel<T, 1, 4, 4>::launch(a, blocks, smem, s);
+    if (p.pb == 1) return EnsKernel<T, 1, 4, ens_minb_mid<T>()>::launch(a, blocks, smem, s);
     return EnsKernel<T, 4, 6, 2>::launch(a, blocks, smem, s);
 }
 

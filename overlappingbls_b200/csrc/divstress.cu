@@ -5,9 +5,9 @@
 
 namespace obl {
 
-// k_cols2 for OP_DERIV on real columns, with the DivEpi store hook
+// The three-radix column unit for OP_DERIV on real columns, with the DivEpi store hook
 template <typename T, int N, int NW, int WB, bool TWG>
-__global__ void __launch_bounds__(32 * NW, col_min_blocks(NW, TWG, col_warps_sm<OP_DERIV>())) k_cols_divt(ColArgs<T> a, DivEpi<T> e)
+__global__ void __launch_bounds__(32 * NW, col_min_blocks(TWG)) k_cols_divt(ColArgs<T> a, DivEpi<T> e)
 {
     using C = C2<T>;
     using D = LineDerived<N, OP_DERIV>;
@@ -30,8 +30,8 @@ template <typename T, int N>
 static cudaError_t launch_divt_n(const ColArgs<T> &a, const DivEpi<T> &e, cudaStream_t s)
 {
     static bool inits[kMaxDevices] = {};
-    constexpr int NW = col_warps<T, N, OP_DERIV>(), WB = col_lines<T, N, OP_DERIV>();
-    constexpr bool TWG = col_tw_global<T, N, OP_DERIV>();
+    constexpr int NW = 8, WB = LmGeo<T>::WB;
+    constexpr bool TWG = col_tw_global<T, N>();
     using D = LineDerived<N, OP_DERIV>;
     const size_t sm = TWG ? sizeof(C2<T>) * (size_t)D::NM * WB : cols2_smem<T, N, OP_DERIV, WB>();
     auto kern = k_cols_divt<T, N, NW, WB, TWG>;

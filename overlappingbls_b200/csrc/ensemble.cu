@@ -17,7 +17,15 @@ bool ens_length_supported(int n)
     return false;
 }
 
-template <typename T> int ens_wb() { return LmGeo<T>::WB; }
+int ens_lines_of(int n)
+{
+    switch (n) {
+#define OBL_C(N) case N: return ens_lines<N>();
+        OBL_ENS_FOR_EACH_N(OBL_C)
+#undef OBL_C
+    }
+    return 1;
+}
 
 // ----------------------------------------------------------------------------- self-test
 // One CTA through the grid barrier with its arrival counter preset: 0 releases at once;
@@ -61,51 +69,26 @@ int ens_barrier_selftest(bool never_released, cudaStream_t s, std::string &err)
 // ----------------------------------------------------------------------------- host side
 template <typename T> long long EnsGeoHost<T>::rows_units(int n, long long npairs)
 {
-    switch (n) {
-#define OBL_C(N)                                                                                         \
-    case N: {                                                                                            \
-        const long long per = 8LL * FwdFusedGeo<T, N>::LPW;                                              \
-        return (npairs + per - 1) / per;                                                                 \
-    }
-        OBL_ENS_FOR_EACH_N(OBL_C)
-#undef OBL_C
-    }
-    return 0;
+    const int w = ens_lines_of(n);
+    return (npairs + w - 1) / w;
 }
 
-template <typename T> long long EnsGeoHost<T>::pinv_rows_units(int n, long long npairs)
-{
-    switch (n) {
-#define OBL_C(N)                                                                                         \
-    case N: {                                                                                            \
-        constexpr int LPW = LineDerived<N, OP_INV>::LPW;                                                 \
-        const long long ngroups = (npairs + LPW - 1) / LPW;                                              \
-        return (4 * ngroups + 7) / 8;                                                                    \
-    }
-        OBL_ENS_FOR_EACH_N(OBL_C)
-#undef OBL_C
-    }
-    return 0;
-}
+template <typename T> long long EnsGeoHost<T>::pinv_rows_units(int n, long long npairs) { return 4 * rows_units(n, npairs); }
 
-template <typename T, int N> static size_t ens_smem_rows()
+template <typename T, int N> static size_t ens_smem_rows() { return TpRows<T, N, ens_lines<N>()>::smem_fwd3_seq; }
+template <typename T, int N, int OP> static size_t ens_smem_col()
 {
-    using GG = FwdFusedGeo<T, N>;
-    return sizeof(C2<T>) * ((size_t)GG::TF + GG::TB + GG::TPB) + GG::row_scr;
+    return sizeof(C2<T>) * (size_t)TpLine<N, OP>::ROWS * ens_lines<N>();
 }
 template <typename T, int N> static size_t ens_smem_cols()
 {
-    size_t m = cols2_smem<T, N, OP_PAD>();
-    m = std::max(m, cols2_smem<T, N, OP_DERIV>());
-    m = std::max(m, cols2_smem<T, N, OP_FWD>());
-    using D = LineDerived<N, OP_INV>;
-    m = std::max(m, sizeof(C2<T>) * ((size_t)D::TB + (size_t)N * LmGeo<T>::WB));
-    return m;
+    return std::max({ens_smem_col<T, N, OP_PAD>(), ens_smem_col<T, N, OP_DERIV>(), ens_smem_col<T, N, OP_FWD>(),
+                     TpPinv<T, N, ens_lines<N>()>::smem});
 }
 template <typename T, int N> static size_t ens_smem_pinv_rows()
 {
-    using D = LineDerived<N, OP_INV>;
-    return sizeof(C2<T>) * ((size_t)D::TB + (size_t)8 * D::LPW * scratch_len(N));
+    using G = TpRows<T, N, ens_lines<N>()>;
+    return sizeof(C2<T>) * (size_t)G::WB * G::LF;
 }
 
 template <typename T> size_t EnsGeoHost<T>::smem(int nx, int ny, int pb, int pe)
@@ -131,7 +114,5 @@ template <typename T> size_t EnsGeoHost<T>::smem(int nx, int ny, int pb, int pe)
 
 template struct EnsGeoHost<float>;
 template struct EnsGeoHost<double>;
-template int ens_wb<float>();
-template int ens_wb<double>();
 
 } // namespace obl

@@ -69,14 +69,17 @@ template <typename T> struct EnsGeoHost {
     // dynamic shared memory of the units of phases [pb, pe)
     static size_t smem(int nx, int ny, int pb, int pe);
 };
-template <typename T> int ens_wb();   // lines per CTA of the line-minor column units
+int ens_lines_of(int n);   // lines per unit of an instance's line transforms of length n
 
-// The kernel over phases [PB, PE) with MINB CTAs per SM.  Instantiated: <0,6,2> (the whole
-// step in one launch) and the register-class split <0,1,2> (rows), <1,4,4> (columns, solve,
-// y-inverse), <4,6,2> (x-inverse + project).
+// The kernel over phases [PB, PE) with MINB CTAs per SM.  Instantiated: <0,6> (the whole
+// step in one launch) and the register-class split <0,1,2> (rows), <1,4> (columns, solve,
+// y-inverse), <4,6,2> (x-inverse + project).  FP64 butterflies need the registers of 2 CTAs
+// per SM (bounded for 4, the 48-instance step took 44.6 instead of 36.4 ms in the split form).
 #ifndef OBL_ENS_MINB
-#define OBL_ENS_MINB 4   // CTAs per SM the one-launch persistent kernel's registers are bounded for
+#define OBL_ENS_MINB 4   // CTAs per SM the FP32 one-launch persistent kernel's registers are bounded for
 #endif
+template <typename T> constexpr int ens_minb() { return sizeof(T) == 8 ? 2 : OBL_ENS_MINB; }
+template <typename T> constexpr int ens_minb_mid() { return sizeof(T) == 8 ? 2 : 4; }
 template <typename T, int PB, int PE, int MINB> struct EnsKernel {
     static cudaError_t attr(size_t smem);
     static int blocks_per_sm(size_t smem);            // CTAs of the kernel resident per SM

@@ -49,83 +49,47 @@ __device__ __forceinline__ bool ens_barrier(unsigned *bar, int *err)
     return ok != 0;
 }
 
-// kinds of plan tables held in shared memory
-enum { K_ROWS = 0, K_PAD, K_DDY, K_FWD, K_PINVC, K_PINVR };
+// Every unit runs on all threads of the CTA with as many lines as they serve.  The barrier
+// in front: the previous unit's last reads of the exchange are done.
+constexpr int kEnsThreads = 256;
+template <int N> constexpr int ens_lines() { return kEnsThreads / TwoPass<N>::R0; }
 
-template <typename T, int N>
-__device__ __forceinline__ void ens_rows(const RowsFwd3Args<T> &a, long long u, C2<T> *sm, int &lk, int &ln)
+template <typename T, int N> __device__ __forceinline__ void ens_rows(const RowsFwd3Args<T> &a, long long u, C2<T> *sm)
 {
-    using GG = FwdFusedGeo<T, N>;
-    C2<T> *twF = sm, *twB = twF + GG::TF, *twPB = twB + GG::TB, *scr = twPB + GG::TPB;
-    if (lk != K_ROWS || ln != N) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < GG::TF; i += blockDim.x) twF[i] = a.twF[i];
-        for (int i = threadIdx.x; i < GG::TB; i += blockDim.x) twB[i] = a.twB[i];
-        for (int i = threadIdx.x; i < GG::TPB; i += blockDim.x) twPB[i] = a.twPB[i];
-        __syncthreads();
-        lk = K_ROWS;
-        ln = N;
-    }
-    rows_fwd3_unit<T, N>(a, u, twF, twB, twPB, scr);
+    __syncthreads();
+    tp_rows_fwd3_unit<T, N, ens_lines<N>(), true>(a, u, sm);
 }
 
 template <typename T, int N, int OP, bool REAL>
-__device__ __forceinline__ void ens_cols(const ColArgs<T> &a, int nb, long long loc, int kind, C2<T> *sm, int &lk,
-                                         int &ln)
+__device__ __forceinline__ void ens_cols(const ColArgs<T> &a, int nb, long long loc, C2<T> *sm)
 {
-    using D = LineDerived<N, OP>;
-    C2<T> *twF = sm, *twB = twF + D::TF, *buf = twB + D::TB;
-    __syncthreads();   // the previous unit's last reads of the exchange scratch are done
-    if (lk != kind || ln != N) {
-        load_tables<T, N, OP>(a.twF, a.twB, twF, twB);
-        __syncthreads();
-        lk = kind;
-        ln = N;
-    }
-    const int z = (int)(loc / nb), bx = (int)(loc - (long long)z * nb);
-    cols2_unit<T, N, OP, REAL>(a, bx, z, twF, twB, buf);
-}
-
-template <typename T, int N>
-__device__ __forceinline__ void ens_pinv_cols(const PinvColArgs<T> &a, int nb, long long loc, C2<T> *sm, int &lk,
-                                              int &ln)
-{
-    using D = LineDerived<N, OP_INV>;
-    C2<T> *twB = sm, *buf = twB + D::TB;
     __syncthreads();
-    if (lk != K_PINVC || ln != N) {
-        for (int i = threadIdx.x; i < D::TB; i += blockDim.x) twB[i] = a.twB[i];
-        __syncthreads();
-        lk = K_PINVC;
-        ln = N;
-    }
     const int z = (int)(loc / nb), bx = (int)(loc - (long long)z * nb);
-    pinv_cols_unit<T, N>(a, bx, z, twB, buf);
+    tp_cols_unit<T, N, OP, REAL, kEnsThreads, ens_lines<N>()>(a, bx, z, sm);
 }
 
 template <typename T, int N>
-__device__ __forceinline__ void ens_pinv_rows(const PinvRowArgs<T> &a, long long u, C2<T> *sm, int &lk, int &ln)
+__device__ __forceinline__ void ens_pinv_cols(const PinvColArgs<T> &a, int nb, long long loc, C2<T> *sm)
 {
-    using D = LineDerived<N, OP_INV>;
-    C2<T> *twB = sm, *scr = twB + D::TB;
-    if (lk != K_PINVR || ln != N) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < D::TB; i += blockDim.x) twB[i] = a.twB[i];
-        __syncthreads();
-        lk = K_PINVR;
-        ln = N;
-    }
-    pinv_rows_unit<T, N>(a, u, twB, scr);
+    __syncthreads();
+    const int z = (int)(loc / nb), u = (int)(loc - (long long)z * nb);
+    tp_pinv_cols_unit<T, N, ens_lines<N>()>(a, u, z, sm);
+}
+
+template <typename T, int N> __device__ __forceinline__ void ens_pinv_rows(const PinvRowArgs<T> &a, long long u, C2<T> *sm)
+{
+    __syncthreads();
+    tp_pinv_rows_unit<T, N, ens_lines<N>()>(a, (int)(u & 3), (u >> 2) * ens_lines<N>(), sm);
 }
 
 template <typename T>
-__device__ __forceinline__ void ens_unit(int ph, const EnsInst<T> &I, long long loc, C2<T> *sm, int &lk, int &ln)
+__device__ __forceinline__ void ens_unit(int ph, const EnsInst<T> &I, long long loc, C2<T> *sm)
 {
     if (ph == 0) {   // multi-output rows: ddx, x-pad, RHS x-spectra
         const int f = (int)(loc / I.rows_units);
         const long long u = loc - (long long)f * I.rows_units;
         switch (I.nx) {
-#define OBL_C(N) case N: ens_rows<T, N>(I.rows[f], u, sm, lk, ln); break;
+#define OBL_C(N) case N: ens_rows<T, N>(I.rows[f], u, sm); break;
             OBL_ENS_FOR_EACH_N(OBL_C)
 #undef OBL_C
         }
@@ -135,7 +99,7 @@ __device__ __forceinline__ void ens_unit(int ph, const EnsInst<T> &I, long long 
             const long long per = (long long)I.pad_nb * I.nlev;
             const int f = (int)(loc / per);
             switch (I.ny) {
-#define OBL_C(N) case N: ens_cols<T, N, OP_PAD, true>(I.padc[f], I.pad_nb, loc - f * per, K_PAD, sm, lk, ln); break;
+#define OBL_C(N) case N: ens_cols<T, N, OP_PAD, true>(I.padc[f], I.pad_nb, loc - f * per, sm); break;
                 OBL_ENS_FOR_EACH_N(OBL_C)
 #undef OBL_C
             }
@@ -143,7 +107,7 @@ __device__ __forceinline__ void ens_unit(int ph, const EnsInst<T> &I, long long 
             const long long per = (long long)I.ddy_nb * I.nlev, l = loc - np;
             const int f = (int)(l / per);
             switch (I.ny) {
-#define OBL_C(N) case N: ens_cols<T, N, OP_DERIV, true>(I.ddyc[f], I.ddy_nb, l - f * per, K_DDY, sm, lk, ln); break;
+#define OBL_C(N) case N: ens_cols<T, N, OP_DERIV, true>(I.ddyc[f], I.ddy_nb, l - f * per, sm); break;
                 OBL_ENS_FOR_EACH_N(OBL_C)
 #undef OBL_C
             }
@@ -151,7 +115,7 @@ __device__ __forceinline__ void ens_unit(int ph, const EnsInst<T> &I, long long 
             const long long per = (long long)I.fwd_nb * I.L, l = loc - np - nd;
             const int f = (int)(l / per);
             switch (I.ny) {
-#define OBL_C(N) case N: ens_cols<T, N, OP_FWD, false>(I.fwdc[f], I.fwd_nb, l - f * per, K_FWD, sm, lk, ln); break;
+#define OBL_C(N) case N: ens_cols<T, N, OP_FWD, false>(I.fwdc[f], I.fwd_nb, l - f * per, sm); break;
                 OBL_ENS_FOR_EACH_N(OBL_C)
 #undef OBL_C
             }
@@ -169,13 +133,13 @@ __device__ __forceinline__ void ens_unit(int ph, const EnsInst<T> &I, long long 
             tdma_column<T, T, false>(I.tdma, I.isl, (loc - I.isl_units) * blockDim.x + threadIdx.x);
     } else if (ph == 3) {   // y-inverse of p_hat and the dpdz spectrum
         switch (I.ny) {
-#define OBL_C(N) case N: ens_pinv_cols<T, N>(I.pc, I.pc_nb, loc, sm, lk, ln); break;
+#define OBL_C(N) case N: ens_pinv_cols<T, N>(I.pc, I.pc_nb, loc, sm); break;
             OBL_ENS_FOR_EACH_N(OBL_C)
 #undef OBL_C
         }
     } else if (ph == 4) {   // x-inverse fused with project()
         switch (I.nx) {
-#define OBL_C(N) case N: ens_pinv_rows<T, N>(I.pr, loc, sm, lk, ln); break;
+#define OBL_C(N) case N: ens_pinv_rows<T, N>(I.pr, loc, sm); break;
             OBL_ENS_FOR_EACH_N(OBL_C)
 #undef OBL_C
         }
@@ -196,11 +160,10 @@ __device__ __forceinline__ void ens_unit(int ph, const EnsInst<T> &I, long long 
 // ~128, the column and solve phases ~64, so the split launches run those at twice the
 // occupancy).
 template <typename T, int PB, int PE, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_ensemble(EnsArgs<T> e)
+__global__ void __launch_bounds__(kEnsThreads, MINB) k_ensemble(EnsArgs<T> e)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     C2<T> *sm = reinterpret_cast<C2<T> *>(smraw);
-    int lk = -1, ln = -1;   // kind and line length of the tables now in shared memory
     auto stamp = [&](int i) {
         if (e.stamps && blockIdx.x == 0 && threadIdx.x == 0) {
             unsigned long long t;
@@ -218,7 +181,7 @@ __global__ void __launch_bounds__(256, MINB) k_ensemble(EnsArgs<T> e)
         int k = 0;
         for (long long it = i0; it < i1; ++it) {
             while (it >= st[k + 1]) ++k;
-            ens_unit<T>(ph, e.inst[k], it - st[k], sm, lk, ln);
+            ens_unit<T>(ph, e.inst[k], it - st[k], sm);
         }
         if (ph + 1 < PE && !ens_barrier(e.bar, e.err)) return;
         stamp(ph + 1);
@@ -253,7 +216,7 @@ __device__ __forceinline__ bool ens_wait_count(const unsigned *cnt, unsigned nee
 constexpr int kEnsFlowSmemInst = 64;
 
 template <typename T, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_ensemble_flow(EnsArgs<T> e)
+__global__ void __launch_bounds__(kEnsThreads, MINB) k_ensemble_flow(EnsArgs<T> e)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     C2<T> *sm = reinterpret_cast<C2<T> *>(smraw);
@@ -263,7 +226,6 @@ __global__ void __launch_bounds__(256, MINB) k_ensemble_flow(EnsArgs<T> e)
     // (instance, phase) pairs this CTA has seen complete, so that their later units skip the
     // check (instances past kEnsFlowSmemInst are always checked)
     __shared__ unsigned char sDone[kEnsFlowSmemInst * kEnsPhases];
-    int lk = -1, ln = -1;   // kind and line length of the tables now in shared memory
     const int n1 = e.ninst + 1;
     const bool cached = e.ninst <= kEnsFlowSmemInst;
     if (cached)
@@ -307,7 +269,7 @@ __global__ void __launch_bounds__(256, MINB) k_ensemble_flow(EnsArgs<T> e)
         }
         __syncthreads();
         if (!sOk) return;
-        ens_unit<T>(ph, I, g - st[k], sm, lk, ln);
+        ens_unit<T>(ph, I, g - st[k], sm);
         __syncthreads();   // every thread's writes of the unit are issued; sOk is read
         // release: the unit's writes (ordered before by the CTA barrier) become visible to a
         // CTA that acquires the count; the reduction does not wait for them

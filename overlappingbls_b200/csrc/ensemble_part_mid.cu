@@ -3,5 +3,5 @@
 
 namespace obl {
 template struct EnsKernel<float, 1, 4, 4>;
-template struct EnsKernel<double, 1, 4, 4>;
+template struct EnsKernel<double, 1, 4, ens_minb_mid<double>()>;
 } // namespace obl

@@ -102,29 +102,24 @@ template <typename T> int FwdFusedLaunch<T>::max_clusters(int n, int csize)
 template struct FwdFusedLaunch<float>;
 template struct FwdFusedLaunch<double>;
 
+template <typename K> static cudaError_t allow_smem(K kern, size_t sm, bool (&inits)[kMaxDevices])
+{
+    const int ds = device_slot();
+    if (ds >= 0 && inits[ds]) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e == cudaSuccess && ds >= 0) inits[ds] = true;
+    return e;
+}
+
 template <typename T, int N> static cudaError_t rows3_run_n(const RowsFwd3Args<T> &a, cudaStream_t s)
 {
-    using GG = FwdFusedGeo<T, N>;
-    const size_t sm = sizeof(C2<T>) * ((size_t)GG::TF + GG::TB + GG::TPB) + GG::row_scr;
-    static int caps[kMaxDevices] = {};
-    auto kern = k_rows_fwd3<T, N>;
-    const int ds = device_slot();
-    int cap = ds >= 0 ? caps[ds] : 0;
-    if (!cap) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        int dev = 0, nsm = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, sm);
-        cap = nsm * (per > 0 ? per : 1);
-        if (ds >= 0) caps[ds] = cap;
-    }
-    const long long per_cta = 8LL * GG::LPW;
-    const long long want = (a.npairs + per_cta - 1) / per_cta;
-    const int grid = (int)(want < cap ? want : cap);
+    using G = TpRows<T, N>;
+    static bool inits[kMaxDevices] = {};
+    cudaError_t e = allow_smem(k_tp_rows_fwd3<T, N>, G::smem_fwd3, inits);
+    if (e != cudaSuccess) return e;
+    const long long grid = (a.npairs + G::WB - 1) / G::WB;
     if (grid < 1) return cudaSuccess;
-    kern<<<grid, 256, sm, s>>>(a);
+    k_tp_rows_fwd3<T, N><<<(unsigned)grid, G::NT, G::smem_fwd3, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -143,48 +138,26 @@ template struct RowsFwd3Launch<double>;
 
 template <typename T, int N> static cudaError_t pinv_cols_n(const PinvColArgs<T> &a, int nlev, cudaStream_t s)
 {
-    using D = LineDerived<N, OP_INV>;
-    // (the 4-CTA shape of the other column kernels measured slower here: the four inverse
-    // transforms of one load need more than its 64 registers)
-    constexpr bool TWG = false;
-    constexpr int NW = TWG ? 8 : col_warps<T, N, OP_INV>();
-    const size_t sm = sizeof(C2<T>) * ((TWG ? 0 : (size_t)D::TB) + (size_t)N * LmGeo<T>::WB);
+    using G = TpPinv<T, N>;
     static bool inits[kMaxDevices] = {};
-    auto kern = k_cols_pinv<T, N, NW, TWG>;
-    const int ds = device_slot();
-    if (ds < 0 || !inits[ds]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        if (ds >= 0) inits[ds] = true;
-    }
-    dim3 grid((a.lhx + LmGeo<T>::WB - 1) / LmGeo<T>::WB, nlev);
-    kern<<<grid, 32 * NW, sm, s>>>(a);
+    cudaError_t e = allow_smem(k_tp_cols_pinv<T, N>, G::smem, inits);
+    if (e != cudaSuccess) return e;
+    const int nbx = (a.lhx + G::WB - 1) / G::WB;
+    dim3 grid(nbx + (nbx + 1) / 2, nlev);
+    k_tp_cols_pinv<T, N><<<grid, G::NT, G::smem, s>>>(a);
     return cudaGetLastError();
 }
 
 template <typename T, int N> static cudaError_t pinv_rows_n(const PinvRowArgs<T> &a, cudaStream_t s)
 {
-    using D = LineDerived<N, OP_INV>;
-    const size_t sm = sizeof(C2<T>) * ((size_t)D::TB + (size_t)8 * D::LPW * scratch_len(N));
-    static int caps[kMaxDevices] = {};
-    auto kern = k_rows_pinv<T, N>;
-    const int ds = device_slot();
-    int cap = ds >= 0 ? caps[ds] : 0;
-    if (!cap) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        int dev = 0, nsm = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, sm);
-        cap = nsm * (per > 0 ? per : 1);
-        if (ds >= 0) caps[ds] = cap;
-    }
-    const long long items = 4 * ((a.npairs + D::LPW - 1) / D::LPW);   // (pair group, component)
-    const long long want = (items + 7) / 8;
-    const int grid = (int)(want < cap ? want : cap);
+    using G = TpRows<T, N>;
+    static bool inits[kMaxDevices] = {};
+    constexpr size_t sm = sizeof(C2<T>) * (size_t)G::WB * G::LF;
+    cudaError_t e = allow_smem(k_tp_rows_pinv<T, N>, sm, inits);
+    if (e != cudaSuccess) return e;
+    const long long grid = 4 * ((a.npairs + G::WB - 1) / G::WB);
     if (grid < 1) return cudaSuccess;
-    kern<<<grid, 256, sm, s>>>(a);
+    k_tp_rows_pinv<T, N><<<(unsigned)grid, G::NTI, sm, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -269,60 +269,135 @@ template <typename T> struct RowsFwd3Args {
     const C2<T> *twF, *twB, *twPB;
 };
 
-// Unit u of the multi-output row pass: warp w of the CTA takes the LPW row pairs from
-// (u*8 + w)*LPW.  Tables in shared memory; scr holds the 8*LPW per-line scratch lines.
-// Called by k_rows_fwd3 (grid-stride over units) and by the persistent ensemble kernel.
-template <typename T, int N>
-__device__ __forceinline__ void rows_fwd3_unit(const RowsFwd3Args<T> &a, long long u, const C2<T> *twF,
-                                               const C2<T> *twB, const C2<T> *twPB, C2<T> *scr)
+// Unit u of the multi-output row pass: the WB row pairs from u*WB.  One forward transform;
+// its spectrum stays in registers (16 values a thread at N = 512) until both backward
+// transforms have made their first pass into exchanges of their own, so that the last
+// passes of ddx and of the padded rows share one phase and no register holds the spectrum
+// through them.
+// SEQ: the two backward transforms share one exchange, one after the other, with the
+// spectrum held through the first (the persistent ensemble kernel, whose CTAs per SM the
+// larger shared memory would cut).
+template <typename T, int N, int WB_ = 0, bool SEQ = false>
+__device__ __forceinline__ void tp_rows_fwd3_unit(const RowsFwd3Args<T> &a, long long u, C2<T> *buf)
 {
     using C = C2<T>;
-    using GG = FwdFusedGeo<T, N>;
-    constexpr int N2 = GG::N2, LH = GG::LH, LPW = GG::LPW;
-    constexpr int LL = GG::DD::LL;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int g = lane / LL, t = lane % LL;
-    C *line = scr + (warp * LPW + g) * scratch_len(N2);
-    {
-        const long long base = (u * nw + warp) * LPW;
-        if (base >= a.npairs) return;
-        const long long p = base + g;
-        const bool act = p < a.npairs;
-        const long long r0 = 2 * (act ? p : base);
-        // warp-uniform: the LPW pairs of a warp lie on one level (ny/2 is a multiple of LPW)
-        const int zw = a.z0 + (int)((2 * base) / a.ny);
-        bool spec = a.H != nullptr && zw >= 1 && zw <= a.L;
-        // checked build: the pair lies in the launch's rows, on one level, and its RHS rows
-        // in H's levels z0..L
-        if (OBL_CHECK && !(ck_in(r0 + 1, 2 * a.npairs, CK_ROWS3_ROW) && ck_in(r0 % a.ny + 1, a.ny, CK_ROWS3_ROW)))
-            return;
-        if (OBL_CHECK && spec && !ck_in(r0 + 1, (long long)(a.L + 1 - a.z0) * a.ny, CK_ROWS3_SPEC)) spec = false;
+    using G = TpRows<T, N, WB_>;
+    constexpr int R0 = G::R0, R1 = G::R1, RP = G::RP, WB = G::WB, NT = G::NT, N2 = G::N2, LH = G::LH;
+    constexpr int LP = G::LPF;      // the forward exchange shares the padded one's memory
+    C *bufP = buf, *bufD = SEQ ? buf : buf + WB * LP;
+    const long long base = u * WB;
+    const int tid = threadIdx.x;
+    auto active = [&](int ln) {
+        const long long p = base + ln;
+        // checked build: the pair lies in the launch's rows and on one level
+        return p < a.npairs && ck_in(2 * p + 1, 2 * a.npairs, CK_ROWS3_ROW) && ck_in((2 * p) % a.ny + 1, a.ny, CK_ROWS3_ROW);
+    };
+    auto src = [&](int ln, const T *&A, const T *&B) {
+        if (!active(ln)) return false;
+        A = a.src + 2 * (base + ln) * a.ldx;
+        B = A + a.ldx;
+        return true;
+    };
+    const T scale = (T)1 / (T)N;
+    tp_rows_first<T, R0, R1, WB, NT, LP>(src, scale, bufP);
+    __syncthreads();
+    const int line = tid / R0, j = tid % R0;
+    C v[R1];
+#pragma unroll
+    for (int r = 0; r < R1; ++r) v[r] = bufP[line * LP + r * G::PF + j];
+#pragma unroll
+    for (int r = 1; r < R1; ++r) v[r] = cmul(v[r], __ldg(a.twF + r * R0 + j));
+    Dft<R1, true>::run(v);                                 // FFT((x - c)/N), bins j + r*R0
+    __syncthreads();                                       // the forward exchange is read
+    // (1) half spectra of the RHS on levels 1..L: FFT(sc*x) = N*sc*v + sc*c*N at DC, x-Nyquist zeroed
+    if (a.H) {
+        const bool act = active(line);
+        const long long r0 = 2 * (base + (act ? line : 0));
+        const int z = a.z0 + (int)(r0 / a.ny);
+        const bool spec = act && z >= 1 && z <= a.L && ck_in(r0 + 1, (long long)(a.L + 1 - a.z0) * a.ny, CK_ROWS3_SPEC);
+        const T s1 = (T)((double)N * a.sc_press), h = (T)0.5 * s1;
+        C *sA = a.H + r0 * LH, *sB = sA + LH;
         const T *A = a.src + r0 * a.ldx;
-        T *dA = a.dfdx + r0 * a.ldx;
-        T *pA = a.xpad + r0 * N2;
-        C *sA = spec ? a.H + r0 * LH : nullptr;
-        C *sB = spec ? a.H + (r0 + 1) * LH : nullptr;
-        row_fwd_fused<T, N>(A, A + a.ldx, dA, dA + a.ldx, pA, pA + N2, sA, sB, act, spec, a.sc_press, a.kx,
-                            twF, twB, twPB, line, t);
+        auto put = [&](int k, C s, C d) {
+            C ao = cscale(s, h), bo = cscale(d, h);
+            if (spec) {
+                if (k == 0) {
+                    ao.x += s1 * A[0];
+                    bo.x += s1 * A[a.ldx];
+                }
+                sA[k] = ao;
+                sB[k] = bo;
+            }
+        };
+        if constexpr (32 % R0 == 0) {
+            tp_split_spectra<T, R0, R1>(v, j, put);
+        } else {
+#pragma unroll
+            for (int r = 0; r < R1; ++r) bufP[line * LP + j + r * R0] = v[r];
+            __syncthreads();
+            tp_split_spectra_smem<T, N, R0, R1>(v, j, bufP + line * LP, put);
+            __syncthreads();
+        }
+        if (spec && j == 0) sA[N / 2] = sB[N / 2] = mk<T>(0, 0);
     }
+    // (2) first passes of the x-pad to 3N/2 (108_01_padd.f90:100-112) and of ddx
+    // (004_derivatives.f90:33-39), (3) their last passes.  The loops of the two last passes
+    // deal their butterflies from opposite ends, so the warps without a padded one start
+    // with ddx
+    auto pad_first = [&]() {
+        if (j == 0) v[R1 / 2] = mk<T>(0, 0);               // the source's Nyquist bin (0 for ddx too)
+        DftPad<R1>::run(v, [&](auto ic, C x) { bufP[line * LP + j * G::PP + decltype(ic)::value] = x; });
+    };
+    auto ddx_first = [&]() {
+        tp_deriv<T, N, R0, R1>(v, a.kx, j);
+        Dft<R1, false>::run(v);
+#pragma unroll
+        for (int r = 0; r < R1; ++r) bufD[line * G::LD + j * G::PD + r] = v[r];
+    };
+    auto pad_last = [&]() {
+        tp_rows_last<T, R0, RP, WB, NT, LP>(tid, bufP, a.twPB, [&](int ln, int jj, const C(&x)[R0]) {
+            if (!active(ln)) return;
+            const long long r0 = 2 * (base + ln);
+            const T ca = a.src[r0 * a.ldx], cb = a.src[(r0 + 1) * a.ldx];
+            T *A = a.xpad + r0 * N2, *B = A + N2;
+#pragma unroll
+            for (int r = 0; r < R0; ++r) {
+                A[jj + r * RP] = x[r].x + ca;
+                B[jj + r * RP] = x[r].y + cb;
+            }
+        });
+    };
+    auto ddx_last = [&]() {
+        tp_rows_last<T, R0, R1, WB, NT, G::LD>(NT - 1 - tid, bufD, a.twB, [&](int ln, int jj, const C(&x)[R0]) {
+            if (!active(ln)) return;
+            T *A = a.dfdx + 2 * (base + ln) * a.ldx, *B = A + a.ldx;
+#pragma unroll
+            for (int r = 0; r < R0; ++r) {
+                A[jj + r * R1] = x[r].x;
+                B[jj + r * R1] = x[r].y;
+            }
+        });
+    };
+    pad_first();
+    if constexpr (SEQ) {
+        __syncthreads();
+        pad_last();
+        __syncthreads();
+        ddx_first();
+        __syncthreads();
+    } else {
+        ddx_first();
+        __syncthreads();
+        pad_last();
+    }
+    ddx_last();
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(256, 2) k_rows_fwd3(RowsFwd3Args<T> a)
+__global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) k_tp_rows_fwd3(RowsFwd3Args<T> a)
 {
-    using C = C2<T>;
-    using GG = FwdFusedGeo<T, N>;
     extern __shared__ __align__(16) unsigned char smraw[];
-    C *twF = reinterpret_cast<C *>(smraw);
-    C *twB = twF + GG::TF;
-    C *twPB = twB + GG::TB;
-    C *scr = twPB + GG::TPB;
-    for (int i = threadIdx.x; i < GG::TF; i += blockDim.x) twF[i] = a.twF[i];
-    for (int i = threadIdx.x; i < GG::TB; i += blockDim.x) twB[i] = a.twB[i];
-    for (int i = threadIdx.x; i < GG::TPB; i += blockDim.x) twPB[i] = a.twPB[i];
-    __syncthreads();
-    const long long per = (long long)(blockDim.x >> 5) * GG::LPW;
-    for (long long u = blockIdx.x; u * per < a.npairs; u += gridDim.x) rows_fwd3_unit<T, N>(a, u, twF, twB, twPB, scr);
+    tp_rows_fwd3_unit<T, N>(a, blockIdx.x, reinterpret_cast<C2<T> *>(smraw));
 }
 
 template <typename T> struct RowsFwd3Launch {
@@ -343,92 +418,90 @@ template <typename T> struct PinvColArgs {
     const C2<T> *twB;
 };
 
-// One CTA unit: line group bx of level z (twB in shared memory, buf = N*WB scratch).
-template <typename T, int N, int NW = 8>
-__device__ __forceinline__ void pinv_cols_unit(const PinvColArgs<T> &a, int bx, int z, const C2<T> *twB, C2<T> *buf)
+// One CTA unit of the y-inverse: two transforms of level z, WB lines each, one middle
+// butterfly per thread.  Units u < nbx take line group u of p_hat and make both of its
+// transforms (p_hat and i*ky*p_hat, one load); the others take two line groups of the dpdz
+// spectrum.  Both transforms make their first passes into exchanges of their own and share
+// the last phase, in which radix-32 butterflies of one line group would leave half of the
+// threads idle.
+template <typename T, int N, int WB_ = 0> struct TpPinv {
+    static constexpr int R0 = TwoPass<N>::R0, R1 = TwoPass<N>::R1, WB = WB_ ? WB_ : TpGeo<T, N, OP_INV>::WB, NT = R0 * WB;
+    static constexpr int PO = tp_pitch(R1), LE = R0 * PO * WB;     // one exchange
+    static constexpr size_t smem = sizeof(C2<T>) * 2 * (size_t)LE;
+    // resident warps per SM (512 lines, 64 levels, FP32: 16 warps 89 us, 24 105 us, the three
+    // radix kernel 103; FP64: 162, 187 before; 128 lines: FP32 29 -> 23, FP64 80 -> 41)
+    static constexpr int wsm = sizeof(T) == 4 ? (R0 >= 24 ? 16 : 24) : (R0 == 32 ? 8 : 12);
+    static constexpr int minb = wsm * 32 / NT > 0 ? wsm * 32 / NT : 1;
+};
+template <typename T, int N, int WB_ = 0>
+__device__ __forceinline__ void tp_pinv_cols_unit(const PinvColArgs<T> &a, int u, int z, C2<T> *buf)
 {
     using C = C2<T>;
-    using D = LineDerived<N, OP_INV>;
-    using G = LmGeo<T, NW>;
-    constexpr int WB = G::WB, LL = G::LL, VR = ColDerived<T, N, OP_INV, NW>::VR;
-    constexpr int R0 = D::RB0, RL = D::RBL;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int line = lane % WB, t = lane / WB + (32 / WB) * warp;
-    const int gl = bx * WB + line;
-    const bool act = gl < a.lhx;
-    const int glc = act ? gl : 0;
-    LineMinor<C, WB> sc{buf, line};
-    using G0 = Geo<N, R0, LL>;
-    using GL = Geo<N, RL, LL>;
-    auto load = [&](const C *src, C *v) {
+    using G = TpPinv<T, N, WB_>;
+    constexpr int R0 = G::R0, R1 = G::R1, WB = G::WB, NT = G::NT, PO = G::PO, LE = G::LE;
+    const int tid = threadIdx.x, line = tid % WB, j = tid / WB;
+    const int nbx = (a.lhx + WB - 1) / WB;
+    const bool pp = u < nbx;                        // p_hat's unit
+    if (!pp && z == 0) return;                      // level 0 needs p only
+    const int g0 = pp ? u : 2 * (u - nbx), g1 = pp ? u : g0 + 1;
+    const int nt = pp ? (z == 0 ? 1 : 2) : (g1 < nbx ? 2 : 1);
+    auto load = [&](const C *src, int g, C(&v)[R1]) {
+        const int gl = g * WB + line;
 #pragma unroll
-        for (int b = 0; b < G0::PER; ++b) {
-            const int j = t + LL * b;
+        for (int r = 0; r < R1; ++r) {
+            const long long q = (long long)(j + r * R0) * a.lhx + gl;
+            v[r] = gl < a.lhx && ck_in(q, a.S, CK_PINV_COL_LOAD) ? __ldcg(src + a.S * z + q) : mk<T>(0, 0);
+        }
+    };
+    auto first = [&](C(&v)[R1], C *b) {
+        Dft<R1, false>::run(v);
+#pragma unroll
+        for (int r = 0; r < R1; ++r) b[(j * PO + r) * WB + line] = v[r];
+    };
+    {
+        C v[R1], w[R1];
+        load(pp ? a.ph : a.dph, g0, v);
+        if (pp) {
+            // i*kx p_hat needs no transform of its own: kx is constant along y, so its
+            // y-inverse is i*kx times that of p_hat, applied by the x-inverse row pass
+#pragma unroll
+            for (int r = 0; r < R1; ++r) {
+                const T kyv = (T)a.ky[j + r * R0];
+                w[r] = mk<T>(-kyv * v[r].y, kyv * v[r].x);
+            }
+        } else if (nt > 1) {
+            load(a.dph, g1, w);
+        }
+        first(v, buf);
+        if (nt > 1) first(w, buf + LE);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int f = tid; f < nt * R1 * WB; f += NT) {
+        const int q = f / (R1 * WB), jj = (f / WB) % R1;
+        const C *b = buf + q * LE;
+        C *dst = pp ? (q == 0 ? a.Xp : a.Xdy) : a.Xdz;
+        const int gl = (q == 0 ? g0 : g1) * WB + line;
+        C x[R0];
+#pragma unroll
+        for (int r = 0; r < R0; ++r) x[r] = b[(r * PO + jj) * WB + line];
+#pragma unroll
+        for (int r = 1; r < R0; ++r) x[r] = cmulc(x[r], __ldg(a.twB + r * R1 + jj));
+        Dft<R0, false>::run(x);
+        if (gl < a.lhx) {
 #pragma unroll
             for (int r = 0; r < R0; ++r) {
-                const int i = j + r * G0::NB;
-                v[b * R0 + r] = (act && (G0::FULL || j < G0::NB) &&
-                                 ck_in((long long)i * a.lhx + glc, a.S, CK_PINV_COL_LOAD))
-                                    ? __ldcg(src + a.S * z + (long long)i * a.lhx + glc)
-                                    : mk<T>(0, 0);
+                const long long i = (long long)(jj + r * R1) * a.lhx + gl;
+                if (ck_in(i, a.S, CK_PINV_COL_STORE)) dst[a.S * z + i] = x[r];
             }
         }
-    };
-    auto store = [&](C *dst, const C *v) {
-        if (!act) return;
-#pragma unroll
-        for (int b = 0; b < GL::PER; ++b) {
-            const int j = t + LL * b;
-            if (GL::FULL || j < GL::NB)
-#pragma unroll
-                for (int r = 0; r < RL; ++r)
-                    if (ck_in((long long)(j + r * GL::NB) * a.lhx + gl, a.S, CK_PINV_COL_STORE))
-                        dst[a.S * z + (long long)(j + r * GL::NB) * a.lhx + gl] = v[b * RL + r];
-        }
-    };
-    C v[VR], w[VR];
-    load(a.ph, v);
-    // i*ky(row) and i*kx(col) multipliers act element-wise on the loaded layout
-#pragma unroll
-    for (int q = 0; q < VR; ++q) w[q] = v[q];
-    fft_regs<N, typename D::PB, LL, false, true>(w, sc, twB, t);
-    store(a.Xp, w);
-    if (z == 0) return;   // uniform per block
-    // i*kx p_hat needs no transform of its own: kx is constant along y, so its y-inverse
-    // is i*kx times that of p_hat, applied by the x-inverse row pass when it loads Xp
-#pragma unroll
-    for (int b = 0; b < G0::PER; ++b) {
-        const int j = t + LL * b;
-#pragma unroll
-        for (int r = 0; r < R0; ++r) {
-            const int i = (G0::FULL || j < G0::NB) ? j + r * G0::NB : 0;
-            const T kyv = (T)a.ky[i];
-            const C x = v[b * R0 + r];
-            w[b * R0 + r] = mk<T>(-kyv * x.y, kyv * x.x);
-        }
     }
-    fft_regs<N, typename D::PB, LL, false, true>(w, sc, twB, t);
-    store(a.Xdy, w);
-    load(a.dph, w);
-    fft_regs<N, typename D::PB, LL, false, true>(w, sc, twB, t);
-    store(a.Xdz, w);
 }
 
-template <typename T, int N, int NW, bool TWG = false>
-__global__ void __launch_bounds__(32 * NW, TWG ? 4 : 2) k_cols_pinv(PinvColArgs<T> a)
+template <typename T, int N> __global__ void __launch_bounds__(TpPinv<T, N>::NT, TpPinv<T, N>::minb) k_tp_cols_pinv(PinvColArgs<T> a)
 {
-    using C = C2<T>;
-    using D = LineDerived<N, OP_INV>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    if constexpr (TWG) {   // twiddles through L1 (see col_tw_global)
-        pinv_cols_unit<T, N, NW>(a, blockIdx.x, blockIdx.y, a.twB, reinterpret_cast<C *>(smraw));
-    } else {
-        C *twB = reinterpret_cast<C *>(smraw);
-        C *buf = twB + D::TB;
-        for (int i = threadIdx.x; i < D::TB; i += blockDim.x) twB[i] = a.twB[i];
-        __syncthreads();
-        pinv_cols_unit<T, N, NW>(a, blockIdx.x, blockIdx.y, twB, buf);
-    }
+    extern __shared__ __align__(128) unsigned char smraw[];
+    tp_pinv_cols_unit<T, N>(a, blockIdx.x, blockIdx.y, reinterpret_cast<C2<T> *>(smraw));
 }
 
 // x-inverse of the four y-inverses and the projection (110_project.f90:16-40) in one
@@ -442,123 +515,96 @@ template <typename T> struct PinvRowArgs {
     long long npairs;                     // ny*(L+1)/2
     int ldx, ny, lhx;
     T dt_tadv1;                           // dt*tadv1
-    const C2<T> *twB;
+    const C2<T> *twF;                     // two-pass table of nx
     int w_from_1;                         // 0: w updated from level 2 (bottom rank, jz_min = 2);
                                           // 1: from level 1 (the z-slab of a rank above it)
 };
 
-// Unit u: warp w takes work item u*8 + w (twB in shared memory, scr = 8*LPW lines).
-template <typename T, int N>
-__device__ __forceinline__ void pinv_rows_unit(const PinvRowArgs<T> &a, long long u, const C2<T> *twB, C2<T> *scr)
+// Unit: component q (0: p; 1: dpdx and u; 2: dpdy and v; 3: dpdz and w) of the WB row pairs
+// from base.
+template <typename T, int N, int WB_ = 0>
+__device__ __forceinline__ void tp_pinv_rows_unit(const PinvRowArgs<T> &a, int q, long long base, C2<T> *buf)
 {
     using C = C2<T>;
-    using D = LineDerived<N, OP_INV>;
-    constexpr int LL = D::LL, LPW = D::LPW, VR = D::VR, R0 = D::RB0, RL = D::RBL;
-    constexpr int SL = scratch_len(N);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int g = lane / LL, t = lane % LL;
-    LineScratch<C> sc{scr + (warp * LPW + g) * SL};
-    using G0 = Geo<N, R0, LL>;
-    using GL = Geo<N, RL, LL>;
+    using G = TpRows<T, N, WB_>;
+    constexpr int R0 = G::R0, R1 = G::R1;
     const long long pl = (long long)a.ldx * a.ny;
-    const long long ngroups = (a.npairs + LPW - 1) / LPW;
-    // work item wi: component q = wi % 4 (0: p; 1: dpdx and u; 2: dpdy and v; 3: dpdz and w)
-    // of the LPW row pairs of group wi / 4.  Independent items keep many row transforms in
-    // flight per SM instead of four dependent ones per warp.
-    {
-        const long long wi = u * nw + warp;
-        if (wi >= 4 * ngroups) return;
-        const int q = (int)(wi % 4);
-        const long long base = (wi / 4) * LPW;
-        const long long pr = base + g;
-        const bool act = pr < a.npairs;
-        const long long r0 = 2 * (act ? pr : base);
-        const int z = (int)((2 * base) / a.ny);            // warp-uniform level
-        if (q > 0 && z == 0) return;                       // level 0 holds p only
+    // levels of the unit's pairs: level 0 holds p only
+    auto row0 = [&](int ln) { return 2 * (base + ln); };
+    auto active = [&](int ln) {
+        const long long p = base + ln;
+        if (p >= a.npairs || (q > 0 && 2 * p < a.ny)) return false;
         // checked build: the pair lies in the launch's rows and on one level
-        if (OBL_CHECK && !(ck_in(r0 + 1, 2 * a.npairs, CK_PINV_ROW) && ck_in(r0 % a.ny + 1, a.ny, CK_PINV_ROW)))
-            return;
-        const long long off = (r0 % a.ny) * a.ldx;
-        const C *X = q <= 1 ? a.Xp : q == 2 ? a.Xdy : a.Xdz;
-        T *out = q == 0 ? a.p + pl * z + off : (q == 1 ? a.dpdx : q == 2 ? a.dpdy : a.dpdz) + pl * (z - 1) + off;
-        T *f = (q == 1 ? a.u : q == 2 ? a.v : a.w) + pl * z + off;
-        const bool proj = q == 1 || q == 2 || (q == 3 && z >= (a.w_from_1 ? 1 : 2));   // jz_min for w
-        // the two rows of the field to update are read before the transform
-        T fa[GL::PER * RL], fb[GL::PER * RL];
+        return ck_in(2 * p + 1, 2 * a.npairs, CK_PINV_ROW) && ck_in((2 * p) % a.ny + 1, a.ny, CK_PINV_ROW);
+    };
+    const C *X = q <= 1 ? a.Xp : q == 2 ? a.Xdy : a.Xdz;
+    auto src = [&](int ln, const C *&A, const C *&B) {
+        if (!active(ln)) return false;
+        A = X + row0(ln) * a.lhx;
+        B = A + a.lhx;
+        return true;
+    };
+    // dpdx: i*kx times the y-inverse of p_hat.  On the two Hermitian rows packed as
+    // Z = A + iB that is i*k_signed*Z (k_signed = kx(k) for bins k <= N/2, -kx(N-k) above)
+    auto op = [&](int j, C(&x)[R0]) {
+        if (q != 1) return;
 #pragma unroll
-        for (int b = 0; b < GL::PER; ++b) {
-            const int j = t + LL * b;
-#pragma unroll
-            for (int r = 0; r < RL; ++r) {
-                const int i = j + r * GL::NB;
-                const bool ok = proj && act && (GL::FULL || j < GL::NB);
-                fa[b * RL + r] = ok ? f[i] : (T)0;
-                fb[b * RL + r] = ok ? f[a.ldx + i] : (T)0;
-            }
+        for (int r = 0; r < R0; ++r) {
+            const int k = j + r * R1;
+            const T kk = k <= N / 2 ? (T)a.kx[k] : -(T)a.kx[N - k];
+            x[r] = mk<T>(-kk * x[r].y, kk * x[r].x);
         }
-        // two Hermitian half spectra (rows r0, r0+1 of X) -> Z = A + iB, Im of DC/Nyquist ignored
-        C v[VR];
-        {
-            const C *A = X + r0 * a.lhx;
-            const C *B = A + a.lhx;
+    };
+    T fa[R1], fb[R1];
+    T *f = nullptr, *out = nullptr;
+    bool act = false, proj = false;
+    // the rows of the field to update are on their way while the exchange is read
+    auto pre = [&](int ln, int j) {
+        act = active(ln);
+        const long long r0 = row0(act ? ln : 0);
+        const int z = (int)(r0 / a.ny);
+        const long long off = (r0 % a.ny) * a.ldx + j;
+        proj = act && (q == 1 || q == 2 || (q == 3 && z >= (a.w_from_1 ? 1 : 2)));   // jz_min for w
+        f = (q == 1 ? a.u : q == 2 ? a.v : a.w) + pl * z + off;
+        out = q == 0 ? a.p + pl * z + off : (q == 1 ? a.dpdx : q == 2 ? a.dpdy : a.dpdz) + pl * (z - 1) + off;
 #pragma unroll
-            for (int b = 0; b < G0::PER; ++b) {
-                const int j = t + LL * b;
-#pragma unroll
-                for (int r = 0; r < R0; ++r) {
-                    const int i = j + r * G0::NB;
-                    C zz = mk<T>(0, 0);
-                    if (act && (G0::FULL || j < G0::NB)) {
-                        const bool lo = i <= N / 2;
-                        const int k = lo ? i : N - i;
-                        C av = __ldcg(A + k), bv = __ldcg(B + k);
-                        if (k == 0 || k == N / 2) { av.y = 0; bv.y = 0; }
-                        zz = lo ? mk<T>(av.x - bv.y, av.y + bv.x) : mk<T>(av.x + bv.y, bv.x - av.y);
-                    }
-                    v[b * R0 + r] = zz;
-                }
-            }
+        for (int r = 0; r < R1; ++r) {
+            fa[r] = proj ? f[r * R0] : (T)0;
+            fb[r] = proj ? f[a.ldx + r * R0] : (T)0;
         }
-        // dpdx: i*kx times the y-inverse of p_hat.  On the two Hermitian rows packed as
-        // Z = A + iB that is i*k_signed*Z (k_signed = kx(k) for bins k <= N/2, -kx(N-k)
-        // above), the multiplier of the x-derivative, applied after the loads
-        if (q == 1) reg_deriv<T, N, R0, LL>(v, a.kx, t);
-        fft_regs<N, typename D::PB, LL, false>(v, sc, twB, t);
-        if (act) {
-#pragma unroll
-            for (int b = 0; b < GL::PER; ++b) {
-                const int j = t + LL * b;
-                if (GL::FULL || j < GL::NB)
-#pragma unroll
-                    for (int r = 0; r < RL; ++r) {
-                        const int i = j + r * GL::NB;
-                        const C x = v[b * RL + r];
-                        out[i] = x.x;
-                        out[a.ldx + i] = x.y;
-                        if (proj) {   // 110_project.f90:16-40: u = u + dt*(-tadv1*dpdx)
-                            f[i] = fa[b * RL + r] + (-a.dt_tadv1 * x.x);
-                            f[a.ldx + i] = fb[b * RL + r] + (-a.dt_tadv1 * x.y);
-                        }
-                    }
-            }
+    };
+    // the update's rows into L2 before the first pass: one 128-byte line per lane
+    if (q > 0) {
+        constexpr int EL = 128 / sizeof(T), PL = (N + EL - 1) / EL;
+        for (int i = threadIdx.x; i < 2 * PL * G::WB; i += G::NTI) {
+            const int ln = i / (2 * PL);
+            if (!active(ln)) continue;
+            const long long r0 = row0(ln);
+            const T *p = (q == 1 ? a.u : q == 2 ? a.v : a.w) + pl * (r0 / a.ny) + (r0 % a.ny + (i / PL) % 2) * a.ldx + (i % PL) * EL;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
         }
     }
+    tp_rows_inv<T, N, WB_>(src, op, buf, a.twF, pre, [&](int, int, const C(&x)[R1]) {
+        if (!act) return;
+#pragma unroll
+        for (int r = 0; r < R1; ++r) {
+            out[r * R0] = x[r].x;
+            out[a.ldx + r * R0] = x[r].y;
+            if (proj) {   // 110_project.f90:16-40: u = u + dt*(-tadv1*dpdx)
+                f[r * R0] = fa[r] + (-a.dt_tadv1 * x[r].x);
+                f[a.ldx + r * R0] = fb[r] + (-a.dt_tadv1 * x[r].y);
+            }
+        }
+    });
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(256, 2) k_rows_pinv(PinvRowArgs<T> a)
+__global__ void __launch_bounds__(TpRows<T, N>::NTI, TpRows<T, N>::minbI) k_tp_rows_pinv(PinvRowArgs<T> a)
 {
-    using C = C2<T>;
-    using D = LineDerived<N, OP_INV>;
     extern __shared__ __align__(16) unsigned char smraw[];
-    C *twB = reinterpret_cast<C *>(smraw);
-    C *scr = twB + D::TB;
-    for (int i = threadIdx.x; i < D::TB; i += blockDim.x) twB[i] = a.twB[i];
-    __syncthreads();
-    const long long ngroups = (a.npairs + D::LPW - 1) / D::LPW;
-    const long long nunits = (4 * ngroups + (blockDim.x >> 5) - 1) / (blockDim.x >> 5);
-    for (long long u = blockIdx.x; u < nunits; u += gridDim.x) pinv_rows_unit<T, N>(a, u, twB, scr);
+    tp_pinv_rows_unit<T, N>(a, blockIdx.x & 3, (long long)(blockIdx.x >> 2) * TpRows<T, N>::WB, reinterpret_cast<C2<T> *>(smraw));
 }
+
 template <typename T> struct PinvLaunch {
     static cudaError_t cols(int n, const PinvColArgs<T> &a, int nlev, cudaStream_t s);
     static cudaError_t rows(int n, const PinvRowArgs<T> &a, cudaStream_t s);

@@ -37,21 +37,21 @@ template <typename T, bool FIRST> struct GSrc {
 };
 
 template <typename T, int N, int NW, int WB, bool TWG, bool FIRST>
-__global__ void __launch_bounds__(32 * NW, col_min_blocks(NW, TWG, col_warps_sm<OP_FWD>())) k_cols_gform(ColArgs<T> a, GSrc<T, FIRST> g)
+__global__ void __launch_bounds__(32 * NW, col_min_blocks(TWG)) k_cols_gform(ColArgs<T> a, GSrc<T, FIRST> g)
 {
     using C = C2<T>;
     using D = LineDerived<N, OP_FWD>;
     extern __shared__ __align__(16) unsigned char smraw[];
     if constexpr (TWG) {
-        cols2_unit<T, N, OP_FWD, false, NW, WB, NoColEpi, false, GSrc<T, FIRST>>(
-            a, blockIdx.x, blockIdx.y, a.twF, a.twB, reinterpret_cast<C *>(smraw), NoColEpi(), nullptr, g);
+        cols2_unit<T, N, OP_FWD, false, NW, WB, NoColEpi, GSrc<T, FIRST>>(
+            a, blockIdx.x, blockIdx.y, a.twF, a.twB, reinterpret_cast<C *>(smraw), NoColEpi(), g);
     } else {
         C *twF = reinterpret_cast<C *>(smraw);
         C *buf = twF + D::TF + D::TB;
         load_tables<T, N, OP_FWD>(a.twF, a.twB, twF, twF + D::TF);
         __syncthreads();
-        cols2_unit<T, N, OP_FWD, false, NW, WB, NoColEpi, false, GSrc<T, FIRST>>(a, blockIdx.x, blockIdx.y, twF,
-                                                                                 twF + D::TF, buf, NoColEpi(), nullptr, g);
+        cols2_unit<T, N, OP_FWD, false, NW, WB, NoColEpi, GSrc<T, FIRST>>(a, blockIdx.x, blockIdx.y, twF,
+                                                                                 twF + D::TF, buf, NoColEpi(), g);
     }
 }
 
@@ -59,8 +59,8 @@ __global__ void __launch_bounds__(32 * NW, col_min_blocks(NW, TWG, col_warps_sm<
 template <typename T, int N, bool FIRST>
 static cudaError_t gform_launch(const ColArgs<T> &a, const GSrc<T, FIRST> &g, cudaStream_t s)
 {
-    constexpr int NW = col_warps<T, N, OP_FWD>(), WB = col_lines<T, N, OP_FWD>();
-    constexpr bool TWG = col_tw_global<T, N, OP_FWD>();
+    constexpr int NW = 8, WB = LmGeo<T>::WB;
+    constexpr bool TWG = col_tw_global<T, N>();
     using D = LineDerived<N, OP_FWD>;
     const size_t sm = TWG ? sizeof(C2<T>) * (size_t)D::NM * WB : cols2_smem<T, N, OP_FWD, WB>();
     auto kern = k_cols_gform<T, N, NW, WB, TWG, FIRST>;

@@ -25,12 +25,14 @@
 #include <vector>
 
 #include "async.cuh"
-#include "fft2.cuh"
+#include "twopass.cuh"
 
 namespace obl {
 
 enum LineOp : int { OP_DERIV = 0, OP_PAD = 1, OP_UNPAD = 2, OP_FWD = 3, OP_INV = 4 };
-enum PlanRole : int { ROLE_FWD = 0, ROLE_BWD = 1, ROLE_PADFWD = 2, ROLE_PADBWD = 3 };
+// twiddle tables of a length: the three-radix plans of fft2.cuh, and (+ ROLE_TP) the
+// two-pass ones of twopass.cuh
+enum PlanRole : int { ROLE_FWD = 0, ROLE_BWD = 1, ROLE_PADFWD = 2, ROLE_PADBWD = 3, ROLE_TP = 4 };
 
 template <typename T> struct RowArgs {
     const void *src;          // real rows (DERIV/PAD/UNPAD/FWD) or complex rows (INV)
@@ -60,7 +62,7 @@ template <typename T> struct ColArgs {
     int kmul;                        // INV: 0 none, 1 multiply by i*kx(col), 2 by i*ky(row)
     int pf_ahead;                    // the unit of plane z also prefetches its input lines of
                                      // plane z + pf_ahead into L2 (0 = none)
-    int tma;                         // FP32 y-pad: input tile by tensor-map copies (k_cols2_tma)
+    int tma;                         // FP32 y-pad: input tile by tensor-map copies (k_tp_cols_tma)
     int *wait_err;                   // set to 1 when such a copy's bounded wait gave up
 };
 
@@ -168,150 +170,6 @@ __device__ __forceinline__ void load_tables(const C2<T> *gF, const C2<T> *gB, C2
         for (int i = threadIdx.x; i < D::TF; i += blockDim.x) sF[i] = gF[i];
     if (OP != OP_FWD)
         for (int i = threadIdx.x; i < D::TB; i += blockDim.x) sB[i] = gB[i];
-}
-
-// One warp processes the LPW row pairs base .. base+LPW-1 (pairs at or beyond a.npairs
-// idle).  twF/twB: the plan twiddle tables in shared memory; scr_warp: the warp's
-// scratch lines (LPW * scratch_len(NM) complex).
-template <typename T, int N, int OP>
-__device__ __forceinline__ void row_unit(const RowArgs<T> &a, long long base, const C2<T> *twF,
-                                         const C2<T> *twB, C2<T> *scr_warp, int lane)
-{
-    using C = C2<T>;
-    using D = LineDerived<N, OP>;
-    constexpr int NI = D::NI, NO = D::NO, LL = D::LL, VR = D::VR;
-    constexpr int SL = scratch_len(D::NM);
-    const int g = lane / LL, t = lane % LL;
-    LineScratch<C> sc{scr_warp + g * SL};
-    {
-        const long long pr = base + g;
-        const bool act = pr < a.npairs;
-        const long long r0 = 2 * (act ? pr : 0);
-        C v[VR];
-        T ca = 0, cb = 0;
-        if constexpr (OP == OP_INV) {
-            // two Hermitian half spectra A (row r0), B (row r0+1) -> Z = A + iB on all N
-            // bins; Im of the DC and Nyquist bins is ignored, as in FFTW's c2r
-            using G = Geo<NO, D::RB0, LL>;
-            const C *A = reinterpret_cast<const C *>(a.src) + r0 * a.src_stride;
-            const C *B = A + a.src_stride;
-#pragma unroll
-            for (int b = 0; b < G::PER; ++b) {
-                const int j = t + LL * b;
-#pragma unroll
-                for (int r = 0; r < D::RB0; ++r) {
-                    const int i = j + r * G::NB;
-                    C z = mk<T>(0, 0);
-                    if (act && (G::FULL || j < G::NB)) {
-                        const bool lo = i <= NO / 2;
-                        const int k = lo ? i : NO - i;
-                        C av = A[k], bv = B[k];
-                        if (k == 0 || k == NO / 2) { av.y = 0; bv.y = 0; }
-                        z = lo ? mk<T>(av.x - bv.y, av.y + bv.x) : mk<T>(av.x + bv.y, bv.x - av.y);
-                    }
-                    v[b * D::RB0 + r] = z;
-                }
-            }
-        } else {
-            using G = Geo<NI, D::RF0, LL>;
-            const T *A = reinterpret_cast<const T *>(a.src) + r0 * a.src_stride;
-            const T *B = A + a.src_stride;
-            if (act) { ca = A[0]; cb = B[0]; }
-#pragma unroll
-            for (int b = 0; b < G::PER; ++b) {
-                const int j = t + LL * b;
-#pragma unroll
-                for (int r = 0; r < D::RF0; ++r) {
-                    const int i = j + r * G::NB;
-                    C z = mk<T>(0, 0);
-                    if (act && (G::FULL || j < G::NB)) z = mk<T>((A[i] - ca) * a.scale, (B[i] - cb) * a.scale);
-                    v[b * D::RF0 + r] = z;
-                }
-            }
-            fft_regs<NI, typename D::PF, LL, true>(v, sc, twF, t);
-        }
-
-        if constexpr (OP == OP_FWD) {
-            // split Z into the half spectra of both rows; zero the x-Nyquist
-            // (203_fftn_mpi.f90:25); the subtracted constants return in the DC bins
-            using G = Geo<NI, D::RFL, LL>;
-#pragma unroll
-            for (int b = 0; b < G::PER; ++b) {
-                const int j = t + LL * b;
-                if (G::FULL || j < G::NB)
-#pragma unroll
-                    for (int r = 0; r < D::RFL; ++r) sc.st(j + r * G::NB, v[b * D::RFL + r]);
-            }
-            __syncwarp();
-            C *Ao = reinterpret_cast<C *>(a.dst) + r0 * a.dst_stride;
-            C *Bo = Ao + a.dst_stride;
-            constexpr int H = NI / 2;
-            for (int k = t; k <= H; k += LL) {
-                C ao = mk<T>(0, 0), bo = mk<T>(0, 0);
-                if (k < H) {
-                    const C z = sc.ld(k), zc = cconj(sc.ld(k == 0 ? 0 : NI - k));
-                    const C s = cadd(z, zc), d = csub(z, zc);
-                    ao = mk<T>((T)0.5 * s.x, (T)0.5 * s.y);
-                    bo = mk<T>((T)0.5 * d.y, (T)-0.5 * d.x);
-                    if (k == 0) {
-                        ao.x += ca * a.scale * (T)NI;
-                        bo.x += cb * a.scale * (T)NI;
-                    }
-                }
-                if (act) {
-                    Ao[k] = ao;
-                    Bo[k] = bo;
-                }
-            }
-            __syncwarp();
-        } else {
-            C w[VR];
-            C *vb = v;
-            if constexpr (OP == OP_DERIV) reg_deriv<T, N, D::RFL, LL>(v, a.ktab, t);
-            if constexpr (OP == OP_PAD) { reg_pad<T, N, D::RFL, LL>(v, w, t); vb = w; }
-            if constexpr (OP == OP_UNPAD) { reg_unpad<T, N, D::RB0, LL>(v, w, t); vb = w; }
-            fft_regs<NO, typename D::PB, LL, false>(vb, sc, twB, t);
-            using G = Geo<NO, D::RBL, LL>;
-            T *A = reinterpret_cast<T *>(a.dst) + r0 * a.dst_stride;
-            T *B = A + a.dst_stride;
-            const T addA = (OP == OP_PAD || OP == OP_UNPAD) ? ca : (T)0;
-            const T addB = (OP == OP_PAD || OP == OP_UNPAD) ? cb : (T)0;
-            if (act) {
-#pragma unroll
-                for (int b = 0; b < G::PER; ++b) {
-                    const int j = t + LL * b;
-                    if (G::FULL || j < G::NB)
-#pragma unroll
-                        for (int r = 0; r < D::RBL; ++r) {
-                            const int i = j + r * G::NB;
-                            A[i] = vb[b * D::RBL + r].x + addA;
-                            B[i] = vb[b * D::RBL + r].y + addB;
-                        }
-                }
-                if (OP == OP_INV && a.pad_mode && t < 2) {
-                    A[NO + t] *= a.pad_scale;
-                    B[NO + t] *= a.pad_scale;
-                }
-            }
-        }
-    }
-}
-
-template <typename T, int N, int OP>
-__global__ void __launch_bounds__(256) k_rows(RowArgs<T> a)
-{
-    using C = C2<T>;
-    using D = LineDerived<N, OP>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    C *twF = reinterpret_cast<C *>(smraw);
-    C *twB = twF + D::TF;
-    C *scr = twB + D::TB;
-    load_tables<T, N, OP>(a.twF, a.twB, twF, twB);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (long long base = ((long long)blockIdx.x * nw + warp) * D::LPW; base < a.npairs;
-         base += (long long)gridDim.x * nw * D::LPW)
-        row_unit<T, N, OP>(a, base, twF, twB, scr + warp * D::LPW * scratch_len(D::NM), lane);
 }
 
 // ----------------------------------------------------------------------------- column kernel
@@ -504,69 +362,15 @@ template <typename T, int NW_ = 8, int WB_ = (sizeof(T) == 4 ? 8 : 4)> struct Lm
     static constexpr int NW = NW_;                        // warps per CTA
     static constexpr int LL = (32 / WB) * NW;             // butterfly slots per line
 };
-// Warps per CTA of the standalone column kernels.  FP32 lines of 256 and more get 16
-// (twice the butterfly slots per line: half the registers per lane and twice the warps per
-// SM at the same shared memory), except the y-pad, which measured fastest with 8; FP64
-// (4 lines per CTA, already 64 slots per line) and the persistent ensemble units use 8.
-#ifndef OBL_PAD_TWG
-#define OBL_PAD_TWG 1
-#endif
-#ifndef OBL_COLS_TWG
-#define OBL_COLS_TWG 1
-#endif
-#ifndef OBL_PAD_NW
-#define OBL_PAD_NW 8
-#endif
-#ifndef OBL_PAD_WB
-#define OBL_PAD_WB 8
-#endif
-#ifndef OBL_COLS_NW
-#define OBL_COLS_NW 8   // warps per CTA of the FP32 ddy / forward y-transform of long lines
-#endif
-#ifndef OBL_COLS_WB
-#define OBL_COLS_WB 8   // lines per CTA of the same
-#endif
+// Shape of the three-radix column kernels that remain beside the two-pass ones below (the G
+// form and the stress divergence, whose load and store hooks hold more registers than a
+// radix-32 butterfly leaves): 8 warps a CTA; FP32 lines of 256 and more read their twiddles
+// through L1, with the registers bounded for 32 warps an SM.
 #ifndef OBL_COL_PF
 #define OBL_COL_PF 2   // y-pad column kernel: L2 prefetch distance in quarters of a residency window (0 = off)
 #endif
-template <typename T, int N, int OP> constexpr int col_warps()
-{
-    return (sizeof(T) == 4 && N >= 256) ? (OP == OP_PAD ? OBL_PAD_NW
-                                                        : ((OBL_COLS_TWG && (OP == OP_DERIV || OP == OP_FWD)) ? OBL_COLS_NW : 16))
-                                        : 8;
-}
-// Twiddles read through L1 instead of staged in shared memory, with the registers bounded
-// for 4 CTAs per SM (4 independent CTAs in different phases of their load / transform /
-// store cycle instead of 3, or 2 of 16 warps).  For the FP32 y-pad of long lines this
-// frees the 11.5 KB of tables that kept it at 3 CTAs per SM: 23% faster.  OBL_COLS_TWG
-// applies the same shape (8 warps) to ddy and the forward y-transform: 24% and 19% faster
-// than 16-warp CTAs with staged tables.
-template <typename T, int N, int OP> constexpr bool col_tw_global()
-{
-    return sizeof(T) == 4 && N >= 256 &&
-           ((OP == OP_PAD && OBL_PAD_TWG) || ((OP == OP_DERIV || OP == OP_FWD) && OBL_COLS_TWG));
-}
-// lines per CTA of the standalone column kernels (build-time knob for the FP32 y-pad)
-template <typename T, int N, int OP> constexpr int col_lines()
-{
-    return (sizeof(T) == 4 && N >= 256 && OP == OP_PAD)
-               ? OBL_PAD_WB
-               : ((sizeof(T) == 4 && N >= 256 && OBL_COLS_TWG && (OP == OP_DERIV || OP == OP_FWD)) ? OBL_COLS_WB
-                                                                                                 : LmGeo<T>::WB);
-}
-// Minimum resident CTAs per SM the column kernels are compiled for: with twiddles through
-// L1, registers are bounded so that the CTAs of 32 warps in total fit on an SM.
-#ifndef OBL_COL_WARPS_SM
-#define OBL_COL_WARPS_SM 32   // resident warps per SM the register bound is set for
-#endif
-#ifndef OBL_COLS_WARPS_SM
-#define OBL_COLS_WARPS_SM OBL_COL_WARPS_SM   // the same for ddy and the y-transform alone
-#endif
-constexpr int col_min_blocks(int nw, bool twg, int warps_sm = OBL_COL_WARPS_SM)
-{
-    return twg ? (nw >= warps_sm ? 1 : warps_sm / nw) : 1;
-}
-template <int OP> constexpr int col_warps_sm() { return (OP == OP_DERIV || OP == OP_FWD) ? OBL_COLS_WARPS_SM : OBL_COL_WARPS_SM; }
+template <typename T, int N> constexpr bool col_tw_global() { return sizeof(T) == 4 && N >= 256; }
+constexpr int col_min_blocks(bool twg) { return twg ? 4 : 1; }
 
 template <typename T, int N, int OP, int NW = 8, int WB = LmGeo<T>::WB> struct ColDerived {
     using D = LineDerived<N, OP>;
@@ -591,14 +395,13 @@ struct NoColSrc {};
 
 // One CTA unit of the line-minor column kernel: line group bx of plane z.  The plan
 // tables twF/twB are already in shared memory; buf is the exchange scratch (NM*WB).
-// Called by k_cols2 (one unit per CTA) and by the persistent ensemble kernel.
-// tile (SMEM_IN): the unit's input already in shared memory, row i of line l at
-// tile[i*WB + l] (the persistent pipelined kernel below); otherwise read from global.
+// Called by the column kernels with hooks (gform.cu, divstress.cu) and by the persistent
+// ensemble kernel.
 template <typename T, int N, int OP, bool REAL, int NW = 8, int WB_ = LmGeo<T>::WB, class EPI = NoColEpi,
-          bool SMEM_IN = false, class SRC = NoColSrc>
+          class SRC = NoColSrc>
 __device__ __forceinline__ void cols2_unit(const ColArgs<T> &a, int bx, int z, const C2<T> *twF,
                                            const C2<T> *twB, C2<T> *buf, const EPI &epi = EPI(),
-                                           const C2<T> *tile = nullptr, const SRC &src = SRC())
+                                           const SRC &src = SRC())
 {
     using C = C2<T>;
     using E = typename std::conditional<REAL, T, C>::type;
@@ -624,7 +427,6 @@ __device__ __forceinline__ void cols2_unit(const ColArgs<T> &a, int bx, int z, c
     };
     auto gld = [&](int i) -> C {
         if constexpr (!std::is_same<SRC, NoColSrc>::value) return src(z, i, glc);
-        else if constexpr (SMEM_IN) return tile[i * WB + line];
         else {
             if (OBL_CHECK && !col_ok(i, glc, a.src_row, a.src_plane, CK_COL_LOAD)) return mk<T>(0, 0);
             if constexpr (REAL) return __ldcg(reinterpret_cast<const C *>(srcz + (long long)i * a.src_row + 2 * glc));
@@ -657,24 +459,6 @@ __device__ __forceinline__ void cols2_unit(const ColArgs<T> &a, int bx, int z, c
                 v[b * D::RF0 + r] = x;
             }
         }
-#if OBL_COL_PF
-        // the CTA that processes this line group pf_ahead planes later (about one
-        // residency window of CTAs) finds its input in L2
-        if (!SMEM_IN && a.pf_ahead > 0 && act && z + a.pf_ahead < a.nlev) {
-            const E *pz = srcz + (long long)a.pf_ahead * a.src_plane;
-#pragma unroll
-            for (int b = 0; b < GG::PER; ++b) {
-                const int j = t + LL * b;
-                if (GG::FULL || j < GG::NB)
-#pragma unroll
-                    for (int r = 0; r < D::RF0; ++r) {
-                        const long long i = j + r * GG::NB;
-                        const E *ptr = pz + i * a.src_row + (REAL ? 2 * glc : glc);
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr));
-                    }
-            }
-        }
-#endif
         if constexpr (!std::is_same<EPI, NoColEpi>::value) {
             using GP = Geo<NO, D::RBL, LL>;
             if (act) {
@@ -687,9 +471,6 @@ __device__ __forceinline__ void cols2_unit(const ColArgs<T> &a, int bx, int z, c
                 }
             }
         }
-        // an input tile in shared memory may be the exchange scratch itself: every thread
-        // has its elements before the first pass stores into it
-        if constexpr (SMEM_IN) __syncthreads();
         fft_regs<NI, typename D::PF, LL, true, true>(v, sc, twF, t);
     }
     if constexpr (OP == OP_FWD) {
@@ -765,87 +546,565 @@ __device__ __forceinline__ void cols2_unit(const ColArgs<T> &a, int bx, int z, c
     }
 }
 
-template <typename T, int N, int OP, bool REAL, int NW, int WB, bool TWG = false>
-__global__ void __launch_bounds__(32 * NW, col_min_blocks(NW, TWG, col_warps_sm<OP>())) k_cols2(ColArgs<T> a)
+// ----------------------------------------------------------------------------- two-pass columns
+// Geometry of a line operation: RI, RO the second radices of its input and output
+// transforms, PI and PO the pitches of their exchanges, ROWS the exchange rows of one line
+// (a forward-only transform takes radix R1 first and exchanges R0 rows of pitch PO).
+template <int N, int OP> struct TpLine {
+    static constexpr int R0 = TwoPass<N>::R0, R1 = TwoPass<N>::R1;
+    static constexpr int RI = OP == OP_UNPAD ? 3 * R1 / 2 : R1, RO = OP == OP_PAD ? 3 * R1 / 2 : R1;
+    static constexpr int NI = R0 * RI, NO = R0 * RO;
+    static constexpr int PI = tp_pitch(R0), PO = tp_pitch(RO);
+    static constexpr int rows_in = OP == OP_INV || OP == OP_FWD ? 0 : RI * PI, rows_out = R0 * PO;
+    static constexpr int ROWS = rows_in > rows_out ? rows_in : rows_out;
+};
+
+// v (bins j + r*R0 of a line of N) *= i*k_signed (ktab[N/2] = 0 drops the Nyquist mode)
+template <typename T, int N, int R0, int R1>
+__device__ __forceinline__ void tp_deriv(C2<T> (&v)[R1], const double *ktab, int j)
 {
-    using C = C2<T>;
-    using D = LineDerived<N, OP>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    if constexpr (TWG) {
-        cols2_unit<T, N, OP, REAL, NW, WB>(a, blockIdx.x, blockIdx.y, a.twF, a.twB, reinterpret_cast<C *>(smraw));
-    } else {
-        C *twF = reinterpret_cast<C *>(smraw);
-        C *twB = twF + D::TF;
-        C *buf = twB + D::TB;
-        load_tables<T, N, OP>(a.twF, a.twB, twF, twB);
-        __syncthreads();
-        cols2_unit<T, N, OP, REAL, NW, WB>(a, blockIdx.x, blockIdx.y, twF, twB, buf);
+#pragma unroll
+    for (int r = 0; r < R1; ++r) {
+        const int k = j + r * R0;
+        const T kk = k <= N / 2 ? (T)ktab[k] : -(T)ktab[N - k];
+        v[r] = mk<T>(-kk * v[r].y, kk * v[r].x);
     }
 }
 
-// ----------------------------------------------------------------------------- pipelined columns
-// Persistent form of k_cols2: each CTA walks units u = blockIdx.x, + gridDim.x, ... (line
-// group u % nbx of plane u / nbx) and, while it transforms unit u, the next unit's input
-// tile (NI rows x WB lines) is already on its way into shared memory with 8-byte cp.async
-// copies (every address of a field row is 8-byte aligned; its 2056-byte pitch at nxt = 512
-// is not the 16-byte multiple a tensor map needs).  Two tiles alternate; the exchange
-// scratch is separate.  The loads of the column kernel then no longer stall its warps.
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool valid)
-{
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    const int n = valid ? 8 : 0;   // 0: the 8 bytes are zero-filled
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(n));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::); }
-
-template <typename T, int N, int OP, bool REAL, int NW, int WB>
-__device__ __forceinline__ void cols_tile_issue(const ColArgs<T> &a, int nbx, int u, C2<T> *tile)
+// One CTA unit: the WB adjacent complex lines (WB real column pairs, or WB complex columns)
+// bx*WB.. of plane z, NT threads.  Thread t serves line t % WB in every pass, so the WB
+// lanes of a butterfly read and store WB adjacent pairs; the exchange is line-minor
+// (element row e of line l at buf[e*WB + l]).
+// SMEM_IN: the unit's input is already in buf, row i of line l at buf[i*WB + l].
+template <typename T, int N, int OP, bool REAL, int NT, int WB, class EPI = NoColEpi, bool SMEM_IN = false,
+          class SRC = NoColSrc>
+__device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z, C2<T> *buf, const EPI &epi = EPI(),
+                                             const SRC &src = SRC())
 {
     using C = C2<T>;
     using E = typename std::conditional<REAL, T, C>::type;
-    constexpr int NI = LineDerived<N, OP>::NI;
-    const int bx = u % nbx, z = u / nbx;
+    using D = TpLine<N, OP>;
+    constexpr int R0 = D::R0, RI = D::RI, RO = D::RO;
+    constexpr int I1 = RI * WB, I2 = R0 * WB, I3 = RO * WB;       // butterflies of the three mappings
+    constexpr int PER1 = (I1 + NT - 1) / NT, PER2 = I2 / NT, PER3 = (I3 + NT - 1) / NT;
+    static_assert(NT % WB == 0 && I2 % NT == 0, "whole butterflies per thread in the middle passes");
+    static_assert(!SMEM_IN || PER1 == 1, "an input tile is read before its exchange overwrites it");
+    const int tid = threadIdx.x, line = tid % WB;
+    const int gl = bx * WB + line;                         // global line index
     const int nlines = REAL ? a.ncols / 2 : a.ncols;
+    const bool act = gl < nlines;
+    const int glc = act ? gl : 0;
     const E *srcz = reinterpret_cast<const E *>(a.src) + (long long)z * a.src_plane;
-    for (int idx = threadIdx.x; idx < NI * WB; idx += 32 * NW) {
-        const int i = idx / WB, l = idx % WB, gl = bx * WB + l;
-        const bool ok = gl < nlines;
-        const E *g = srcz + (long long)i * a.src_row + (REAL ? 2 * (ok ? gl : 0) : (ok ? gl : 0));
-        cp_async8(tile + idx, g, ok);
+    E *dstz = reinterpret_cast<E *>(a.dst) + (long long)z * a.dst_plane;
+    // the checked build tests each element's level, column and plane offset against the
+    // extents the arguments give (nlev planes of src_plane / dst_plane, rows of src_row / dst_row)
+    auto col_ok = [&](int i, int col, int row, long long plane, int site) {
+        const int ce = REAL ? 2 * col + 1 : col;
+        return ck_in(z, a.nlev, site) && ck_in(ce, row, site) && ck_in((long long)i * row + ce, plane, site);
+    };
+    auto gld = [&](int i) -> C {
+        if constexpr (!std::is_same<SRC, NoColSrc>::value) return src(z, i, glc);
+        else if constexpr (SMEM_IN) return buf[i * WB + line];
+        else {
+            if (OBL_CHECK && !col_ok(i, glc, a.src_row, a.src_plane, CK_COL_LOAD)) return mk<T>(0, 0);
+            if constexpr (REAL) return __ldcg(reinterpret_cast<const C *>(srcz + (long long)i * a.src_row + 2 * glc));
+            else return __ldcg(srcz + (long long)i * a.src_row + glc);
+        }
+    };
+    auto gst = [&](int i, C v) {
+        if (OBL_CHECK && !col_ok(i, gl, a.dst_row, a.dst_plane, CK_COL_STORE)) return;
+        if constexpr (REAL) *reinterpret_cast<C *>(dstz + (long long)i * a.dst_row + 2 * gl) = v;
+        else dstz[(long long)i * a.dst_row + gl] = v;
+    };
+    if constexpr (OP == OP_FWD) {
+        // forward only: radix R1 first, so that every thread loads; twB's table is w_N^(r k),
+        // k < R1
+        constexpr int PF = tp_pitch(D::R1);
+#pragma unroll
+        for (int b = 0; b < PER2; ++b) {
+            const int j = (tid + b * NT) / WB;
+            C x[D::R1];
+#pragma unroll
+            for (int r = 0; r < D::R1; ++r) x[r] = act ? cscale(gld(j + r * R0), a.scale) : mk<T>(0, 0);
+            Dft<D::R1, true>::run(x);
+#pragma unroll
+            for (int r = 0; r < D::R1; ++r) buf[(j * PF + r) * WB + line] = x[r];
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int f = tid; f < D::R1 * WB; f += NT) {
+            const int j = f / WB;
+            C x[R0];
+#pragma unroll
+            for (int r = 0; r < R0; ++r) x[r] = buf[(r * PF + j) * WB + line];
+#pragma unroll
+            for (int r = 1; r < R0; ++r) x[r] = cmul(x[r], __ldg(a.twB + r * D::R1 + j));
+            Dft<R0, true>::run(x);
+            if (act) {
+#pragma unroll
+                for (int r = 0; r < R0; ++r)
+                    gst(j + r * D::R1, r == R0 / 2 && a.zero_nyq && j == 0 ? mk<T>(0, 0) : x[r]);   // bin N/2
+            }
+        }
+        return;
+    }
+    C cref = mk<T>(0, 0);
+    C v[PER2][D::R1];
+
+    if constexpr (OP != OP_INV) {
+        if constexpr (REAL) cref = gld(0);
+#pragma unroll
+        for (int b = 0; b < PER1; ++b) {
+            const int f = tid + b * NT, j = f / WB;
+            const bool on = I1 % NT == 0 || f < I1;
+            C x[R0];
+            if (on) {
+#pragma unroll
+                for (int r = 0; r < R0; ++r)
+                    x[r] = act ? cscale(csub(gld(j + r * RI), cref), a.scale) : mk<T>(0, 0);
+            }
+            if constexpr (SMEM_IN) __syncthreads();   // the tile is read before the exchange overwrites it
+            if (on) {
+                Dft<R0, true>::run(x);
+#pragma unroll
+                for (int r = 0; r < R0; ++r) buf[(j * D::PI + r) * WB + line] = x[r];
+            }
+        }
+        if constexpr (!std::is_same<EPI, NoColEpi>::value) {
+            if (act) {
+#pragma unroll
+                for (int b = 0; b < PER3; ++b) {
+                    const int f = tid + b * NT, j = f / WB;
+                    if (I3 % NT == 0 || f < I3)
+#pragma unroll
+                        for (int r = 0; r < R0; ++r) epi.prefetch(z, j + r * RO, gl);
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < PER2; ++b) {
+            const int j = (tid + b * NT) / WB;
+            C x[RI];
+#pragma unroll
+            for (int r = 0; r < RI; ++r) x[r] = buf[(r * D::PI + j) * WB + line];
+#pragma unroll
+            for (int r = 1; r < RI; ++r) x[r] = cmul(x[r], __ldg(a.twF + r * R0 + j));
+            if constexpr (OP == OP_UNPAD) {
+                DftUnpad<D::R1>::run(x, v[b]);
+                if (j == 0) v[b][RO / 2] = mk<T>(0, 0);   // bin N/2
+            } else {
+                Dft<RI, true>::run(x);
+#pragma unroll
+                for (int r = 0; r < RI; ++r) v[b][r] = x[r];
+            }
+        }
+        if constexpr (OP != OP_FWD) __syncthreads();   // the exchange is read before it is written again
+    } else {
+#pragma unroll
+        for (int b = 0; b < PER2; ++b) {
+            const int j = (tid + b * NT) / WB;
+#pragma unroll
+            for (int r = 0; r < RO; ++r) {
+                const int i = j + r * R0;
+                C x = act ? gld(i) : mk<T>(0, 0);
+                if (a.kmul) {
+                    const T kk = (T)(a.kmul == 1 ? a.ktab[glc] : a.ktab[i]);
+                    x = mk<T>(-kk * x.y, kk * x.x);
+                }
+                v[b][r] = cscale(x, a.scale);
+            }
+        }
+    }
+    if constexpr (OP == OP_FWD) {
+        if (act) {
+#pragma unroll
+            for (int b = 0; b < PER2; ++b) {
+                const int j = (tid + b * NT) / WB;
+#pragma unroll
+                for (int r = 0; r < RI; ++r) {
+                    const int i = j + r * R0;
+                    C x = v[b][r];
+                    if (r == RI / 2 && a.zero_nyq && j == 0) x = mk<T>(0, 0);   // bin N/2
+                    gst(i, x);
+                }
+            }
+        }
+    } else {
+#pragma unroll
+        for (int b = 0; b < PER2; ++b) {
+            const int j = (tid + b * NT) / WB;
+            if constexpr (OP == OP_PAD) {
+                if (j == 0) v[b][RI / 2] = mk<T>(0, 0);   // the source's Nyquist bin
+                DftPad<D::R1>::run(v[b], [&](auto ic, C x) { buf[(j * D::PO + decltype(ic)::value) * WB + line] = x; });
+            } else {
+                if constexpr (OP == OP_DERIV) tp_deriv<T, N, R0, RO>(v[b], a.ktab, j);
+                Dft<RO, false>::run(v[b]);
+#pragma unroll
+                for (int r = 0; r < RO; ++r) buf[(j * D::PO + r) * WB + line] = v[b][r];
+            }
+        }
+        __syncthreads();
+        constexpr bool addc = OP == OP_PAD || OP == OP_UNPAD;
+#pragma unroll 1
+        for (int f = tid; f < I3; f += NT) {
+            const int j = f / WB;
+            C x[R0];
+#pragma unroll
+            for (int r = 0; r < R0; ++r) x[r] = buf[(r * D::PO + j) * WB + line];
+#pragma unroll
+            for (int r = 1; r < R0; ++r) x[r] = cmulc(x[r], __ldg(a.twB + r * RO + j));
+            Dft<R0, false>::run(x);
+            if (act) {
+#pragma unroll
+                for (int r = 0; r < R0; ++r) {
+                    const int i = j + r * RO;
+                    C y = x[r];
+                    if (addc) {
+                        y.x += cref.x;
+                        y.y += cref.y;
+                    }
+                    epi(z, i, gl, y);
+                    gst(i, y);
+                    if constexpr (OP == OP_UNPAD && REAL) {
+                        // var(nxt+1:ldx,:) = var(1:2,:) (108_01_padd.f90:195)
+                        if (a.pad_copy && gl == 0 && ck_in(a.ncols + 1, a.dst_row, CK_COL_STORE))
+                            *reinterpret_cast<C *>(dstz + (long long)i * a.dst_row + a.ncols) = y;
+                    }
+                }
+            }
+        }
     }
 }
 
-template <typename T, int N, int OP, bool REAL, int NW, int WB>
-__global__ void __launch_bounds__(32 * NW, 2) k_cols2_pipe(ColArgs<T> a, int nbx)
+// Threads, lines and registers of the column kernels: WB lines (64-byte row segments; 128
+// bytes for the short lines of R0 = 8), R0*WB/PER2 threads.  FP32: 24 resident warps with
+// one middle butterfly a thread (80 registers) beat 16 warps with two (y-pad of 512 lines,
+// 258 levels: 0.846 against 0.881 ms over four fields; 20 warps spill: 0.949), except
+// where all threads load at once in the forward-only transform (0.351 against 0.388 ms for
+// three spectra).  FP64 radix-32 butterflies need 8 warps; two middle butterflies a thread
+// keep more of them loading (ddy 1.214 against 1.450 ms), which the y-pad's larger exchange
+// does not repay (2.63 against 2.34 ms).
+// Against the three-radix kernels (ms per step at 512x512x256 levels, before -> now): FP32
+// y-pad 1.243 -> 0.846, ddy 0.714 -> 0.571, y-transform 0.393 -> 0.351; FP64 3.00 -> 2.34,
+// 1.85 -> 1.21; at 128x128 levels the y-pad takes 0.62 and the y-unpad 0.55 of their time.
+// The L1/shared pipe fell from 70 to 55% busy at half the time per byte.  A persistent form
+// with the next tile's copies in flight measured slower (1.25 ms): its second tile leaves
+// shared memory for 16 warps only.
+#ifndef OBL_TP_WARPS_SM
+#define OBL_TP_WARPS_SM 24   // resident warps per SM the FP32 column kernels' registers are bounded for
+#endif
+#ifndef OBL_TP_LINES
+#define OBL_TP_LINES 8       // lines per CTA of the FP32 column kernels with R0 > 8
+#endif
+template <typename T, int N, int OP> struct TpGeo {
+    static constexpr int R0 = TwoPass<N>::R0;
+    static constexpr int WB = sizeof(T) == 4 ? (R0 == 8 ? 16 : OBL_TP_LINES) : (R0 == 8 ? 8 : 4);
+    static constexpr int PER2 = R0 == 32 && (OP == OP_FWD || (sizeof(T) == 8 && OP != OP_PAD)) ? 2 : 1;
+    static constexpr int NT = R0 * WB / PER2;
+    static constexpr int wsm = sizeof(T) == 4 ? (PER2 == 2 ? 16 : OBL_TP_WARPS_SM) : (R0 == 32 ? 8 : R0 >= 20 ? 12 : 16);
+    static constexpr int minb = wsm * 32 / NT > 0 ? wsm * 32 / NT : 1;
+};
+template <typename T, int N, int OP> inline size_t tp_cols_smem()
+{
+    using D = TpLine<N, OP>;
+    return sizeof(C2<T>) * (size_t)(D::ROWS > D::NI ? D::ROWS : D::NI) * TpGeo<T, N, OP>::WB;
+}
+template <typename T, int N, int OP, bool REAL>
+__global__ void __launch_bounds__(TpGeo<T, N, OP>::NT, TpGeo<T, N, OP>::minb) k_tp_cols(ColArgs<T> a)
+{
+    using G = TpGeo<T, N, OP>;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    tp_cols_unit<T, N, OP, REAL, G::NT, G::WB>(a, blockIdx.x, blockIdx.y, reinterpret_cast<C2<T> *>(smraw));
+}
+
+// ----------------------------------------------------------------------------- two-pass rows
+// The same two passes for contiguous lines: a CTA holds WB row pairs (each one complex
+// line) and in every pass deals the pairs (line, butterfly) to consecutive threads with the
+// butterfly fastest, so that a warp reads and stores consecutive elements of a row.  The
+// exchange of a line is contiguous; line pitches are 8 modulo 16 elements, which keeps the
+// lines that share a warp on different banks.  Twiddles come through the read-only path.
+// Against the three-radix warp-per-line kernels (us, before -> now, 64 levels of 512x512
+// points or as many points): ddx of 512 lines FP32 52 -> 43, x-unpad 81 -> 68; of 384 lines
+// 54 -> 39, 91 -> 60; FP64 256 lines 94 -> 60, 189 -> 109.
+constexpr int tp_line(int n) { return n + (24 - n % 16) % 16; }
+
+template <typename T, int N, int WB_ = 0> struct TpRows {
+    static constexpr int R0 = TwoPass<N>::R0, R1 = TwoPass<N>::R1, RP = 3 * R1 / 2;
+    static constexpr int N2 = R0 * RP, LH = N / 2 + 1;
+    static constexpr int PF = tp_pitch(R0), PD = tp_pitch(R1), PP = tp_pitch(RP);
+    // exchange elements of one line: forward of N and of 3N/2, backward of N and of 3N/2
+    static constexpr int LF = tp_line(R1 * PF), LF2 = tp_line(RP * PF), LD = tp_line(R0 * PD), LP = tp_line(R0 * PP);
+    static constexpr int WB = WB_ ? WB_ : R0 == 8 ? (sizeof(T) == 4 ? 16 : 8) : R0 == 16 ? (sizeof(T) == 4 ? 8 : 4) : R0 == 20 ? 8 : 4;
+    static constexpr int NT = R0 * WB;                     // one middle-pass butterfly a thread
+    // the inverse's first pass loads: at R0 = 32 its 10..20 butterflies a line are dealt to
+    // half as many threads, which then take two middle butterflies each
+    static constexpr int PERI = R0 == 32 ? 2 : 1, NTI = NT / PERI;
+    // resident warps per SM the registers are bounded for.  FP32: 16 with radices from 20 (20
+    // warps spill: the multi-output pass of 512 lines 1.133 instead of 1.108 ms per step), 20
+    // below; FP64: 8 with radix 32 (12 spill: 3.6 against 2.4 ms), 16 with 20, else 12.
+    static constexpr int wsm = sizeof(T) == 4 ? (R0 >= 20 ? 16 : 20) : (R0 == 32 ? 8 : R0 == 20 ? 16 : 12);
+    static constexpr int minb = wsm * 32 / NT > 0 ? wsm * 32 / NT : 1, minbI = wsm * 32 / NTI > 0 ? wsm * 32 / NTI : 1;
+    static_assert(NT % 32 == 0, "whole warps: the spectra are split by shuffles");
+    template <int OP> static constexpr int line_elems()
+    {
+        return OP == OP_DERIV ? (LF > LD ? LF : LD) : OP == OP_PAD ? (LF > LP ? LF : LP) : OP == OP_UNPAD ? (LF2 > LD ? LF2 : LD)
+                                                                             : OP == OP_FWD ? LF : LF;
+    }
+    static constexpr int LPF = LP > LF ? LP : LF;
+    static constexpr size_t smem_fwd3 = sizeof(C2<T>) * (size_t)WB * (LD + LPF), smem_fwd3_seq = sizeof(C2<T>) * (size_t)WB * LPF;
+};
+
+// First forward pass: butterfly f = (line, j) of radix R0 over x[j + r*RI] of rows A, B
+template <typename T, int R0, int RI, int WB, int NT, int LS, class ROWS>
+__device__ __forceinline__ void tp_rows_first(const ROWS &rows, T scale, C2<T> *buf)
 {
     using C = C2<T>;
-    using D = LineDerived<N, OP>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    C *tile0 = reinterpret_cast<C *>(smraw);
-    C *tile1 = tile0 + D::NI * WB;
-    C *buf = tile1 + D::NI * WB;
-    const int nunits = nbx * a.nlev;
-    int u = blockIdx.x;
-    if (u >= nunits) return;
-    cols_tile_issue<T, N, OP, REAL, NW, WB>(a, nbx, u, tile0);
-    cp_async_commit();
-    for (int it = 0; u < nunits; ++it, u += gridDim.x) {
-        C *cur = (it & 1) ? tile1 : tile0;
-        C *nxt = (it & 1) ? tile0 : tile1;
-        const int un = u + gridDim.x;
-        if (un < nunits) cols_tile_issue<T, N, OP, REAL, NW, WB>(a, nbx, un, nxt);
-        cp_async_commit();
-        cp_async_wait_prev();
-        __syncthreads();
-        cols2_unit<T, N, OP, REAL, NW, WB, NoColEpi, true>(a, u % nbx, u / nbx, a.twF, a.twB, buf, NoColEpi(), cur);
-        __syncthreads();
+#pragma unroll 1
+    for (int f = threadIdx.x; f < RI * WB; f += NT) {
+        const int line = f / RI, j = f % RI;
+        const T *A, *B;
+        if (!rows(line, A, B)) continue;
+        const T ca = A[0], cb = B[0];
+        C x[R0];
+#pragma unroll
+        for (int r = 0; r < R0; ++r) x[r] = mk<T>(A[j + r * RI], B[j + r * RI]);
+        const C c = mk<T>(ca, cb);
+#pragma unroll
+        for (int r = 0; r < R0; ++r) x[r] = cscale(csub(x[r], c), scale);
+        Dft<R0, true>::run(x);
+#pragma unroll
+        for (int r = 0; r < R0; ++r) buf[line * LS + j * tp_pitch(R0) + r] = x[r];
     }
 }
 
-#ifndef OBL_COL_PIPE
-#define OBL_COL_PIPE 0   // FP32 y-pad, ddy and y-transform of long lines: persistent prefetching form
-#endif
+// Last backward pass: butterfly (line, j) of radix R0 from the exchange; emit(line, i, x).
+// `first` is the thread's first butterfly (two loops of one phase start from opposite ends)
+template <typename T, int R0, int RO, int WB, int NT, int LS, class EMIT>
+__device__ __forceinline__ void tp_rows_last(int first, const C2<T> *buf, const C2<T> *tw, EMIT &&emit)
+{
+    using C = C2<T>;
+#pragma unroll 1
+    for (int f = first; f < RO * WB; f += NT) {
+        const int line = f / RO, j = f % RO;
+        C x[R0];
+#pragma unroll
+        for (int r = 0; r < R0; ++r) x[r] = buf[line * LS + r * tp_pitch(RO) + j];
+#pragma unroll
+        for (int r = 1; r < R0; ++r) x[r] = cmulc(x[r], __ldg(tw + r * RO + j));
+        Dft<R0, false>::run(x);
+        emit(line, j, x);
+    }
+}
+
+// Half spectra of the two rows of a line from its spectrum Z (v[r] = bin j + r*R0 in the
+// thread of butterfly j): A = (Z[k] + conj Z[N-k])/2, B = (Z[k] - conj Z[N-k])/(2i) for
+// k < N/2.  Bin N-k is v[R1-1-r] of butterfly R0-j (of the same one for j = 0), a lane of
+// the same warp; emit(k, a, b).  Every lane of the warp calls it.
+template <typename T, int R0, int R1, class EMIT>
+__device__ __forceinline__ void tp_split_spectra(const C2<T> (&v)[R1], int j, EMIT &&emit)
+{
+    using C = C2<T>;
+    static_assert(32 % R0 == 0, "a line's butterflies lie in one warp");
+    const int lane = threadIdx.x & 31, src = (lane & ~(R0 - 1)) + ((R0 - j) & (R0 - 1));
+#pragma unroll
+    for (int r = 0; r < R1 / 2; ++r) {
+        const C p = j == 0 ? v[(R1 - r) % R1] : v[R1 - 1 - r];
+        C q;
+        q.x = __shfl_sync(0xffffffffu, p.x, src);
+        q.y = -__shfl_sync(0xffffffffu, p.y, src);
+        const C s = cadd(v[r], q), d = csub(v[r], q);
+        emit(j + r * R0, s, mk<T>(d.y, -d.x));
+    }
+}
+
+// The same from the line's spectrum in shared memory (bin k at z[k]), for R0 not a power of two
+template <typename T, int N, int R0, int R1, class EMIT>
+__device__ __forceinline__ void tp_split_spectra_smem(const C2<T> (&v)[R1], int j, const C2<T> *z, EMIT &&emit)
+{
+    using C = C2<T>;
+#pragma unroll
+    for (int r = 0; r < R1 / 2; ++r) {
+        const int k = j + r * R0;
+        const C q = cconj(z[k == 0 ? 0 : N - k]);
+        const C s = cadd(v[r], q), d = csub(v[r], q);
+        emit(k, s, mk<T>(d.y, -d.x));
+    }
+}
+
+
+// Inverse of two rows' half spectra A, B (one complex line Z = A + iB on all N bins; Im of
+// the DC and Nyquist bins is ignored, as in FFTW's c2r): radix R0 from global memory, one
+// exchange, radix R1; op(j, z) may multiply the bins j + r*R1 before the transform, and
+// pre(line, j) is called before, emit(line, j, x) with the elements j + r*R0.  tw: the forward table of N = R0*R1
+template <typename T, int N, int WB_, class ROWS, class OPF, class PRE, class EMIT>
+__device__ __forceinline__ void tp_rows_inv(const ROWS &rows, const OPF &op, C2<T> *buf, const C2<T> *tw, PRE &&pre, EMIT &&emit)
+{
+    using C = C2<T>;
+    using G = TpRows<T, N, WB_>;
+    constexpr int R0 = G::R0, R1 = G::R1, WB = G::WB, NT = G::NTI, LS = G::LF;
+#pragma unroll 1
+    for (int f = threadIdx.x; f < R1 * WB; f += NT) {
+        const int line = f / R1, j = f % R1;
+        const C *A, *B;
+        if (!rows(line, A, B)) continue;
+        C x[R0];
+#pragma unroll
+        for (int r = 0; r < R0; ++r) {
+            const int i = j + r * R1;
+            const bool lo = r < R0 / 2 || (r == R0 / 2 && j == 0);   // i <= N/2
+            const int k = lo ? i : N - i;
+            C av = __ldcg(A + k), bv = __ldcg(B + k);
+            if (j == 0 && (r == 0 || r == R0 / 2)) { av.y = 0; bv.y = 0; }
+            x[r] = lo ? mk<T>(av.x - bv.y, av.y + bv.x) : mk<T>(av.x + bv.y, bv.x - av.y);
+        }
+        op(j, x);
+        Dft<R0, false>::run(x);
+#pragma unroll
+        for (int r = 0; r < R0; ++r) buf[line * LS + j * G::PF + r] = x[r];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int b = 0; b < G::PERI; ++b) {
+        const int f = threadIdx.x + b * NT, line = f / R0, j = f % R0;
+        pre(line, j);
+        C x[R1];
+#pragma unroll
+        for (int r = 0; r < R1; ++r) x[r] = buf[line * LS + r * G::PF + j];
+#pragma unroll
+        for (int r = 1; r < R1; ++r) x[r] = cmulc(x[r], __ldg(tw + r * R0 + j));
+        Dft<R1, false>::run(x);
+        emit(line, j, x);
+    }
+}
+
+template <typename T, int N, int OP>
+__device__ __forceinline__ void tp_row_unit(const RowArgs<T> &a, long long base, C2<T> *buf)
+{
+    using C = C2<T>;
+    using G = TpRows<T, N>;
+    constexpr int R0 = G::R0, R1 = G::R1, WB = G::WB, NT = G::NT;
+    constexpr int RI = OP == OP_UNPAD ? G::RP : R1, RO = OP == OP_PAD ? G::RP : R1, NO = R0 * RO;
+    constexpr int LI = OP == OP_UNPAD ? G::LF2 : G::LF, LO = OP == OP_PAD ? G::LP : G::LD;
+    const int tid = threadIdx.x;
+    auto active = [&](int line) { return base + line < a.npairs; };
+    if constexpr (OP != OP_INV) {
+        auto src = [&](int line, const T *&A, const T *&B) {
+            if (!active(line)) return false;
+            A = reinterpret_cast<const T *>(a.src) + 2 * (base + line) * a.src_stride;
+            B = A + a.src_stride;
+            return true;
+        };
+        tp_rows_first<T, R0, RI, WB, NT, LI>(src, a.scale, buf);
+        __syncthreads();
+        const int line = tid / R0, j = tid % R0;
+        C v[R1];
+        {
+            C x[RI];
+#pragma unroll
+            for (int r = 0; r < RI; ++r) x[r] = buf[line * LI + r * G::PF + j];
+#pragma unroll
+            for (int r = 1; r < RI; ++r) x[r] = cmul(x[r], __ldg(a.twF + r * R0 + j));
+            if constexpr (OP == OP_UNPAD) {
+                DftUnpad<R1>::run(x, v);
+                if (j == 0) v[R1 / 2] = mk<T>(0, 0);   // bin N/2
+            } else {
+                Dft<RI, true>::run(x);
+#pragma unroll
+                for (int r = 0; r < RI; ++r) v[r] = x[r];
+            }
+        }
+        if constexpr (OP == OP_FWD) {
+            // both rows' half spectra; the x-Nyquist is zeroed (203_fftn_mpi.f90:25) and the
+            // subtracted constants return in the DC bins.  A[0] and B[0] are read by the
+            // thread that overwrites them when the call transforms in place
+            const bool act = active(line);
+            const long long r0 = 2 * (act ? base + line : base);
+            C *Ao = reinterpret_cast<C *>(a.dst) + r0 * a.dst_stride, *Bo = Ao + a.dst_stride;
+            const T *A = reinterpret_cast<const T *>(a.src) + r0 * a.src_stride;
+            auto put = [&](int k, C s, C d) {
+                C ao = cscale(s, (T)0.5), bo = cscale(d, (T)0.5);
+                if (act) {
+                    if (k == 0) {
+                        ao.x += A[0] * a.scale * (T)N;
+                        bo.x += A[a.src_stride] * a.scale * (T)N;
+                    }
+                    Ao[k] = ao;
+                    Bo[k] = bo;
+                }
+            };
+            if constexpr (32 % R0 == 0) {
+                tp_split_spectra<T, R0, R1>(v, j, put);
+            } else {
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < R1; ++r) buf[line * LI + j + r * R0] = v[r];
+                __syncthreads();
+                tp_split_spectra_smem<T, N, R0, R1>(v, j, buf + line * LI, put);
+            }
+            if (act && j == 0) Ao[N / 2] = Bo[N / 2] = mk<T>(0, 0);
+            return;
+        }
+        __syncthreads();   // the exchange is read before it is written again
+        if constexpr (OP == OP_PAD) {
+            if (j == 0) v[R1 / 2] = mk<T>(0, 0);   // the source's Nyquist bin
+            DftPad<R1>::run(v, [&](auto ic, C x) { buf[line * LO + j * tp_pitch(RO) + decltype(ic)::value] = x; });
+        } else {
+            if constexpr (OP == OP_DERIV) tp_deriv<T, N, R0, R1>(v, a.ktab, j);
+            Dft<R1, false>::run(v);
+#pragma unroll
+            for (int r = 0; r < R1; ++r) buf[line * LO + j * tp_pitch(RO) + r] = v[r];
+        }
+        __syncthreads();
+        constexpr bool addc = OP == OP_PAD || OP == OP_UNPAD;
+        tp_rows_last<T, R0, RO, WB, NT, LO>(tid, buf, a.twB, [&](int ln, int jj, const C(&x)[R0]) {
+            if (!active(ln)) return;
+            const long long r0 = 2 * (base + ln);
+            T *A = reinterpret_cast<T *>(a.dst) + r0 * a.dst_stride, *B = A + a.dst_stride;
+            T addA = 0, addB = 0;
+            if (addc) {
+                const T *S = reinterpret_cast<const T *>(a.src) + r0 * a.src_stride;
+                addA = S[0];
+                addB = S[a.src_stride];
+            }
+#pragma unroll
+            for (int r = 0; r < R0; ++r) {
+                A[jj + r * RO] = x[r].x + addA;
+                B[jj + r * RO] = x[r].y + addB;
+            }
+        });
+    } else {
+        auto src = [&](int line, const C *&A, const C *&B) {
+            if (!active(line)) return false;
+            A = reinterpret_cast<const C *>(a.src) + 2 * (base + line) * a.src_stride;
+            B = A + a.src_stride;
+            return true;
+        };
+        auto same = [](int, C *) {};
+        tp_rows_inv<T, N, 0>(src, same, buf, a.twF, [](int, int) {}, [&](int ln, int jj, const C(&x)[R1]) {
+            const long long r0 = 2 * (base + ln);
+            if (!active(ln)) return;
+            T *A = reinterpret_cast<T *>(a.dst) + r0 * a.dst_stride, *B = A + a.dst_stride;
+#pragma unroll
+            for (int r = 0; r < R1; ++r) {
+                A[jj + r * R0] = x[r].x;
+                B[jj + r * R0] = x[r].y;
+            }
+            if (a.pad_mode && jj < 2) {
+                A[NO + jj] *= a.pad_scale;
+                B[NO + jj] *= a.pad_scale;
+            }
+        });
+    }
+}
+
+template <typename T, int N, int OP>
+__global__ void __launch_bounds__(OP == OP_INV ? TpRows<T, N>::NTI : TpRows<T, N>::NT, OP == OP_INV ? TpRows<T, N>::minbI : TpRows<T, N>::minb)
+    k_tp_rows(RowArgs<T> a)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    tp_row_unit<T, N, OP>(a, (long long)blockIdx.x * TpRows<T, N>::WB, reinterpret_cast<C2<T> *>(smraw));
+}
 
 // ----------------------------------------------------------------------------- TMA-fed y-pad
 // The FP32 y-pad with its CTA's input tile (NI rows x WB real column pairs of the x-padded
@@ -855,15 +1114,16 @@ __global__ void __launch_bounds__(32 * NW, 2) k_cols2_pipe(ColArgs<T> a, int nbx
 // the exchange scratch), completing on an mbarrier, and the same thread asks L2 for the
 // tile pf_ahead planes later (cp.async.bulk.prefetch.tensor).  The tile lands in the
 // exchange scratch the CTA already holds, so shared memory per CTA and CTAs per SM stay
-// those of k_cols2.  The tensor map covers this GPU's own x-padded planes; no multicast.
+// those of k_tp_cols.  The tensor map covers this GPU's own x-padded planes; no multicast.
 // The wait is bounded: on timeout wait_err is set (the host reports OBL_ERR_TIMEOUT), the
 // CTA waits once more (bounded) for the copy, and its results are not to be used.
-template <typename T, int N, int OP, bool REAL, int NW, int WB>
-__global__ void __launch_bounds__(32 * NW, col_min_blocks(NW, true, col_warps_sm<OP>()))
-    k_cols2_tma(ColArgs<T> a, const __grid_constant__ CUtensorMap tm, int box_rows)
+template <typename T, int N, int OP, bool REAL>
+__global__ void __launch_bounds__(TpGeo<T, N, OP>::NT, TpGeo<T, N, OP>::minb)
+    k_tp_cols_tma(ColArgs<T> a, const __grid_constant__ CUtensorMap tm, int box_rows)
 {
     using C = C2<T>;
-    using D = LineDerived<N, OP>;
+    using D = TpLine<N, OP>;
+    constexpr int WB = TpGeo<T, N, OP>::WB;
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ __align__(8) unsigned long long bar;
     // tensor copies write 128-byte aligned shared memory (an offset from smraw keeps the
@@ -894,7 +1154,7 @@ __global__ void __launch_bounds__(32 * NW, col_min_blocks(NW, true, col_warps_sm
         if (a.wait_err) atomicExch(a.wait_err, 1);
         mbar_wait_bounded(sbar, 0);   // a late copy lands before the tile is reused
     }
-    cols2_unit<T, N, OP, REAL, NW, WB, NoColEpi, true>(a, blockIdx.x, blockIdx.y, a.twF, a.twB, buf, NoColEpi(), buf);
+    tp_cols_unit<T, N, OP, REAL, TpGeo<T, N, OP>::NT, WB, NoColEpi, true>(a, blockIdx.x, blockIdx.y, buf);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link)
@@ -929,42 +1189,21 @@ constexpr int tma_box_rows(int ni)
 }
 
 // ----------------------------------------------------------------------------- launchers
-template <typename T, int N, int OP> inline size_t rows_smem()
-{
-    using D = LineDerived<N, OP>;
-    return sizeof(C2<T>) * ((size_t)D::TF + D::TB + (size_t)8 * D::LPW * scratch_len(D::NM));
-}
-template <typename T, int N, int OP, bool REAL> inline size_t cols_smem()
-{
-    using D = LineDerived<N, OP>;
-    using E = typename std::conditional<REAL, T, C2<T>>::type;
-    using TT = ColTile<T, REAL, D::LPW>;
-    return sizeof(C2<T>) * ((size_t)D::TF + D::TB) + sizeof(E) * (size_t)tile_rows(D::NM) * TT::S;
-}
-
 template <typename T, int N, int OP> cudaError_t launch_rows_t(const RowArgs<T> &a, cudaStream_t s)
 {
-    static int caps[kMaxDevices] = {};
-    const size_t sm = rows_smem<T, N, OP>();
-    auto kern = k_rows<T, N, OP>;
+    using G = TpRows<T, N>;
+    static bool inits[kMaxDevices] = {};
+    constexpr size_t sm = sizeof(C2<T>) * (size_t)G::WB * G::template line_elems<OP>();
+    auto kern = k_tp_rows<T, N, OP>;
     const int ds = device_slot();
-    int grid_cap = ds >= 0 ? caps[ds] : 0;
-    if (!grid_cap) {
+    if (ds < 0 || !inits[ds]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
-        int dev = 0, nsm = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, sm);
-        grid_cap = nsm * (per > 0 ? per : 1);
-        if (ds >= 0) caps[ds] = grid_cap;
+        if (ds >= 0) inits[ds] = true;
     }
-    constexpr int LPW = LineDerived<N, OP>::LPW;
-    const long long per_cta = 8LL * LPW;
-    long long want = (a.npairs + per_cta - 1) / per_cta;
-    int grid = (int)(want < grid_cap ? want : grid_cap);
+    const long long grid = (a.npairs + G::WB - 1) / G::WB;
     if (grid < 1) return cudaSuccess;
-    kern<<<grid, 256, sm, s>>>(a);
+    kern<<<(unsigned)grid, OP == OP_INV ? G::NTI : G::NT, sm, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -976,27 +1215,20 @@ template <typename T, int N, int OP, int WB = LmGeo<T>::WB> inline size_t cols2_
 
 template <typename T, int N, int OP, bool REAL> cudaError_t launch_cols_t(const ColArgs<T> &a0, cudaStream_t s)
 {
-    static int residents[kMaxDevices] = {};   // CTAs of this kernel resident on the whole GPU
-    constexpr int NW = col_warps<T, N, OP>(), WB = col_lines<T, N, OP>();
-    constexpr bool TWG = col_tw_global<T, N, OP>();
-    using D = LineDerived<N, OP>;
-    const size_t sm = TWG ? sizeof(C2<T>) * (size_t)D::NM * WB : cols2_smem<T, N, OP, WB>();
-    auto kern = k_cols2<T, N, OP, REAL, NW, WB, TWG>;
+    static bool inits[kMaxDevices] = {};
+    constexpr int WB = TpGeo<T, N, OP>::WB, NT = TpGeo<T, N, OP>::NT;
+    using D = TpLine<N, OP>;
+    const size_t sm = tp_cols_smem<T, N, OP>();
+    auto kern = k_tp_cols<T, N, OP, REAL>;
     const int ds = device_slot();
-    int resident = ds >= 0 ? residents[ds] : 0;
-    if (!resident) {
+    if (ds < 0 || !inits[ds]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
-        int dev = 0, nsm = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 32 * NW, sm);
-        resident = nsm * (per > 0 ? per : 1);
-        if (ds >= 0) residents[ds] = resident;
+        if (ds >= 0) inits[ds] = true;
     }
     ColArgs<T> a = a0;
     const int nlines = REAL ? a.ncols / 2 : a.ncols;
-    if constexpr (std::is_same<T, float>::value && OP == OP_PAD && REAL && TWG && tma_box_rows(D::NI) > 0) {
+    if constexpr (std::is_same<T, float>::value && OP == OP_PAD && REAL && D::RI <= D::R0 && N >= 256 && tma_box_rows(D::NI) > 0) {
         // the x-padded planes as a 2-D map: ncols floats wide (pitch src_row), NI*nlev rows
         const bool fits = a.tma && a.src_plane == a.src_row * (long long)D::NI && (a.src_row * 4) % 16 == 0 &&
                           ((uintptr_t)a.src % 16) == 0 && tensor_map_encoder() != nullptr;
@@ -1012,7 +1244,7 @@ template <typename T, int N, int OP, bool REAL> cudaError_t launch_cols_t(const 
                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return cudaErrorInvalidValue;
             static int tres[kMaxDevices] = {};
-            auto tk = k_cols2_tma<T, N, OP, REAL, NW, WB>;
+            auto tk = k_tp_cols_tma<T, N, OP, REAL>;
             const size_t tsm = sm + 128;
             int tr = ds >= 0 ? tres[ds] : 0;
             if (!tr) {
@@ -1021,44 +1253,20 @@ template <typename T, int N, int OP, bool REAL> cudaError_t launch_cols_t(const 
                 int dev = 0, nsm = 0, per = 0;
                 cudaGetDevice(&dev);
                 cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, tk, 32 * NW, tsm);
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, tk, NT, tsm);
                 tr = nsm * (per > 0 ? per : 1);
                 if (ds >= 0) tres[ds] = tr;
             }
             dim3 grid((nlines + WB - 1) / WB, a.nlev);
             if (grid.x < 1 || grid.y < 1) return cudaSuccess;
             if (OBL_COL_PF) a.pf_ahead = (int)((OBL_COL_PF * (long long)tr + 4LL * grid.x - 1) / (4LL * grid.x));
-            tk<<<grid, 32 * NW, tsm, s>>>(a, tm, BR);
+            tk<<<grid, NT, tsm, s>>>(a, tm, BR);
             return cudaGetLastError();
         }
     }
-    if constexpr (OBL_COL_PIPE && TWG && OP != OP_INV) {
-        static int pres[kMaxDevices] = {};
-        auto pk = k_cols2_pipe<T, N, OP, REAL, NW, WB>;
-        const size_t psm = sizeof(C2<T>) * ((size_t)2 * D::NI * WB + (size_t)D::NM * WB);
-        int pr = ds >= 0 ? pres[ds] : 0;
-        if (!pr) {
-            cudaError_t e = cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
-            if (e != cudaSuccess) return e;
-            int dev = 0, nsm = 0, per = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, pk, 32 * NW, psm);
-            pr = nsm * (per > 0 ? per : 1);
-            if (ds >= 0) pres[ds] = pr;
-        }
-        const int nbx = (nlines + WB - 1) / WB;
-        const long long nunits = (long long)nbx * a.nlev;
-        if (nunits < 1) return cudaSuccess;
-        const int grid = (int)(nunits < pr ? nunits : pr);
-        pk<<<grid, 32 * NW, psm, s>>>(a, nbx);
-        return cudaGetLastError();
-    }
     dim3 grid((nlines + WB - 1) / WB, a.nlev);
-    // y-pad only: measured 5% faster at 512x512x256; ddy and the y-transform did not gain
-    if (OBL_COL_PF && OP == OP_PAD) a.pf_ahead = (int)((OBL_COL_PF * (long long)resident + 4LL * grid.x - 1) / (4LL * grid.x));
     if (grid.x < 1 || grid.y < 1) return cudaSuccess;
-    kern<<<grid, 32 * NW, sm, s>>>(a);
+    kern<<<grid, NT, sm, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -97,6 +97,10 @@ template <int N> std::vector<double> plan_table_n(int role)
     case ROLE_BWD: return plan_table_for(N, PlanVec<BwdPlan<N>>::get());
     case ROLE_PADFWD: return plan_table_for(3 * N / 2, PlanVec<PadFwdPlan<N>>::get());
     case ROLE_PADBWD: return plan_table_for(3 * N / 2, PlanVec<PadBwdPlan<N>>::get());
+    case ROLE_TP + ROLE_FWD: return plan_table_for(N, {TwoPass<N>::R0, TwoPass<N>::R1});
+    case ROLE_TP + ROLE_BWD: return plan_table_for(N, {TwoPass<N>::R1, TwoPass<N>::R0});
+    case ROLE_TP + ROLE_PADFWD: return plan_table_for(3 * N / 2, {TwoPass<N>::R0, 3 * TwoPass<N>::R1 / 2});
+    case ROLE_TP + ROLE_PADBWD: return plan_table_for(3 * N / 2, {3 * TwoPass<N>::R1 / 2, TwoPass<N>::R0});
     }
     return {};
 }

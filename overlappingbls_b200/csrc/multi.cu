@@ -6,74 +6,44 @@
 namespace obl {
 
 template <typename T, int N, int OP>
-__global__ void __launch_bounds__(256) k_rows_multi(RowArgs<T> a0, MultiPtr<T> m, int nf, long long npf)
+__global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) k_tp_rows_multi(RowArgs<T> a0, MultiPtr<T> m, int nb)
 {
-    using C = C2<T>;
-    using D = LineDerived<N, OP>;
     extern __shared__ __align__(16) unsigned char smraw[];
-    C *twF = reinterpret_cast<C *>(smraw);
-    C *twB = twF + D::TF;
-    C *scr = twB + D::TB;
-    load_tables<T, N, OP>(a0.twF, a0.twB, twF, twB);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // npf: each field's pairs rounded up to whole warps' groups, so a group never spans fields
-    for (long long base = ((long long)blockIdx.x * nw + warp) * D::LPW; base < npf * nf;
-         base += (long long)gridDim.x * nw * D::LPW) {
-        const int f = (int)(base / npf);
-        RowArgs<T> a = a0;
-        a.src = m.src[f];
-        a.dst = m.dst[f];
-        row_unit<T, N, OP>(a, base - f * npf, twF, twB, scr + warp * D::LPW * scratch_len(D::NM), lane);
-    }
+    const int f = blockIdx.x / nb;   // nb CTAs per field
+    RowArgs<T> a = a0;
+    a.src = m.src[f];
+    a.dst = m.dst[f];
+    tp_row_unit<T, N, OP>(a, (long long)(blockIdx.x - f * nb) * TpRows<T, N>::WB, reinterpret_cast<C2<T> *>(smraw));
 }
 
-template <typename T, int N, int OP, bool REAL, int NW, int WB, bool TWG>
-__global__ void __launch_bounds__(32 * NW, col_min_blocks(NW, TWG, col_warps_sm<OP>())) k_cols2_multi(ColArgs<T> a0, MultiPtr<T> m)
+template <typename T, int N, int OP, bool REAL>
+__global__ void __launch_bounds__(TpGeo<T, N, OP>::NT, TpGeo<T, N, OP>::minb) k_tp_cols_multi(ColArgs<T> a0, MultiPtr<T> m)
 {
-    using C = C2<T>;
-    using D = LineDerived<N, OP>;
-    extern __shared__ __align__(16) unsigned char smraw[];
+    using G = TpGeo<T, N, OP>;
+    extern __shared__ __align__(128) unsigned char smraw[];
     const int f = blockIdx.y / a0.nlev, z = blockIdx.y - f * a0.nlev;
     ColArgs<T> a = a0;
     a.src = m.src[f];
     a.dst = m.dst[f];
-    if constexpr (TWG) {
-        cols2_unit<T, N, OP, REAL, NW, WB>(a, blockIdx.x, z, a.twF, a.twB, reinterpret_cast<C *>(smraw));
-    } else {
-        C *twF = reinterpret_cast<C *>(smraw);
-        C *twB = twF + D::TF;
-        C *buf = twB + D::TB;
-        load_tables<T, N, OP>(a.twF, a.twB, twF, twB);
-        __syncthreads();
-        cols2_unit<T, N, OP, REAL, NW, WB>(a, blockIdx.x, z, twF, twB, buf);
-    }
+    tp_cols_unit<T, N, OP, REAL, G::NT, G::WB>(a, blockIdx.x, z, reinterpret_cast<C2<T> *>(smraw));
 }
 
 template <typename T, int N, int OP>
 static cudaError_t rows_multi_t(const RowArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
 {
-    static int caps[kMaxDevices] = {};
-    const size_t sm = rows_smem<T, N, OP>();
-    auto kern = k_rows_multi<T, N, OP>;
+    using G = TpRows<T, N>;
+    static bool inits[kMaxDevices] = {};
+    constexpr size_t sm = sizeof(C2<T>) * (size_t)G::WB * G::template line_elems<OP>();
+    auto kern = k_tp_rows_multi<T, N, OP>;
     const int ds = device_slot();
-    int cap = ds >= 0 ? caps[ds] : 0;
-    if (!cap) {
+    if (ds < 0 || !inits[ds]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
-        int dev = 0, nsm = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, sm);
-        cap = nsm * (per > 0 ? per : 1);
-        if (ds >= 0) caps[ds] = cap;
+        if (ds >= 0) inits[ds] = true;
     }
-    constexpr int LPW = LineDerived<N, OP>::LPW;
-    const long long npf = (a.npairs + LPW - 1) / LPW * LPW;
-    const long long want = (npf * nf + 8LL * LPW - 1) / (8LL * LPW);
-    const int grid = (int)(want < cap ? want : cap);
-    if (grid < 1) return cudaSuccess;
-    kern<<<grid, 256, sm, s>>>(a, m, nf, npf);
+    const long long nb = (a.npairs + G::WB - 1) / G::WB;
+    if (nb < 1) return cudaSuccess;
+    kern<<<(unsigned)(nb * nf), G::NT, sm, s>>>(a, m, (int)nb);
     return cudaGetLastError();
 }
 
@@ -81,11 +51,9 @@ template <typename T, int N, int OP, bool REAL>
 static cudaError_t cols_multi_t(const ColArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
 {
     static bool inits[kMaxDevices] = {};
-    constexpr int NW = col_warps<T, N, OP>(), WB = col_lines<T, N, OP>();
-    constexpr bool TWG = col_tw_global<T, N, OP>();
-    using D = LineDerived<N, OP>;
-    const size_t sm = TWG ? sizeof(C2<T>) * (size_t)D::NM * WB : cols2_smem<T, N, OP, WB>();
-    auto kern = k_cols2_multi<T, N, OP, REAL, NW, WB, TWG>;
+    constexpr int WB = TpGeo<T, N, OP>::WB, NT = TpGeo<T, N, OP>::NT;
+    const size_t sm = tp_cols_smem<T, N, OP>();
+    auto kern = k_tp_cols_multi<T, N, OP, REAL>;
     const int ds = device_slot();
     if (ds < 0 || !inits[ds]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -97,7 +65,7 @@ static cudaError_t cols_multi_t(const ColArgs<T> &a, const MultiPtr<T> &m, int n
     const int nlines = REAL ? b.ncols / 2 : b.ncols;
     dim3 grid((nlines + WB - 1) / WB, (unsigned)(b.nlev * nf));
     if (grid.x < 1 || grid.y < 1) return cudaSuccess;
-    kern<<<grid, 32 * NW, sm, s>>>(b, m);
+    kern<<<grid, NT, sm, s>>>(b, m);
     return cudaGetLastError();
 }
 

@@ -10,8 +10,8 @@
 // of fft2.cuh.
 //
 // What bounds the line kernels is the shared-memory/L1 data pipe, which the three-radix
-// kernels kept 75-83% busy at 50% instruction issue and 35% of HBM; an exchange costs a
-// store and a load of every element there.
+// kernels kept 68-76% busy at 50% instruction issue and 21-34% of HBM (512x512x64, FP32);
+// an exchange costs a store and a load of every element there.
 //
 // The lines of a CTA share its threads: in every pass the (butterfly, line) pairs are dealt
 // to consecutive threads, so a pass with fewer butterflies than threads leaves whole warps
@@ -22,7 +22,10 @@
 
 namespace obl {
 
-// N = R0*R1: R0 a multiple of 8 and R1 even (the 3/2 rule's split)
+// N = R0*R1, R1 even (the 3/2 rule's split), R0 a multiple of 4.  The splits keep the two
+// radices within a factor of two, so that no pass leaves most threads without a butterfly:
+// 320 as 20*16 took 43 us for the ddy of 102 levels, as 32*10 66 us, and 384 as 24*16 44 us,
+// as 32*12 62 us.
 template <int N> struct TwoPass;
 template <> struct TwoPass<32> { static constexpr int R0 = 8, R1 = 4; };
 template <> struct TwoPass<48> { static constexpr int R0 = 8, R1 = 6; };
@@ -32,10 +35,10 @@ template <> struct TwoPass<96> { static constexpr int R0 = 8, R1 = 12; };
 template <> struct TwoPass<128> { static constexpr int R0 = 16, R1 = 8; };
 template <> struct TwoPass<160> { static constexpr int R0 = 16, R1 = 10; };
 template <> struct TwoPass<192> { static constexpr int R0 = 16, R1 = 12; };
-template <> struct TwoPass<240> { static constexpr int R0 = 24, R1 = 10; };
+template <> struct TwoPass<240> { static constexpr int R0 = 20, R1 = 12; };
 template <> struct TwoPass<256> { static constexpr int R0 = 16, R1 = 16; };
-template <> struct TwoPass<320> { static constexpr int R0 = 32, R1 = 10; };
-template <> struct TwoPass<384> { static constexpr int R0 = 32, R1 = 12; };
+template <> struct TwoPass<320> { static constexpr int R0 = 20, R1 = 16; };
+template <> struct TwoPass<384> { static constexpr int R0 = 24, R1 = 16; };
 template <> struct TwoPass<512> { static constexpr int R0 = 32, R1 = 16; };
 template <> struct TwoPass<640> { static constexpr int R0 = 32, R1 = 20; };
 

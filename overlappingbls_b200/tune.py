@@ -99,10 +99,9 @@ def step_candidates(nxt, nyt):
 # library as built without definitions.
 BUILD_CANDIDATES = {
     "default": [],
-    "cols_4w4l": ["OBL_PAD_NW=4", "OBL_PAD_WB=4", "OBL_COLS_NW=4", "OBL_COLS_WB=4"],
-    "cols_16w_32sm": ["OBL_PAD_NW=16", "OBL_COLS_NW=16"],
-    "cols_16w_48sm": ["OBL_PAD_NW=16", "OBL_COLS_NW=16", "OBL_COL_WARPS_SM=48"],
-    "cols_pipelined": ["OBL_COL_PIPE=1"],
+    "cols_4w4l": ["OBL_TP_LINES=4"],
+    "cols_16w_sm": ["OBL_TP_WARPS_SM=16"],
+    "cols_32w_sm": ["OBL_TP_WARPS_SM=32"],
     "rows_pad16": ["OBL_SIDX_SHIFT=4"],
     "pad_prefetch_off": ["OBL_COL_PF=0"],
 }
