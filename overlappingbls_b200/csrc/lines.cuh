@@ -625,7 +625,9 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
             const int j = (tid + b * NT) / WB;
             C x[D::R1];
 #pragma unroll
-            for (int r = 0; r < D::R1; ++r) x[r] = act ? cscale(gld(j + r * R0), a.scale) : mk<T>(0, 0);
+            for (int r = 0; r < D::R1; ++r) x[r] = act ? gld(j + r * R0) : mk<T>(0, 0);
+#pragma unroll
+            for (int r = 0; r < D::R1; ++r) x[r] = cscale(x[r], a.scale);
             Dft<D::R1, true>::run(x);
 #pragma unroll
             for (int r = 0; r < D::R1; ++r) buf[(j * PF + r) * WB + line] = x[r];
@@ -660,8 +662,11 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
             C x[R0];
             if (on) {
 #pragma unroll
-                for (int r = 0; r < R0; ++r)
-                    x[r] = act ? cscale(csub(gld(j + r * RI), cref), a.scale) : mk<T>(0, 0);
+                for (int r = 0; r < R0; ++r) x[r] = act ? gld(j + r * RI) : mk<T>(0, 0);
+                // (a loop of its own: arithmetic inside the conditional load kept the loads
+                // from being issued together; ddy of 512 lines 0.669 -> 0.566 ms per step)
+#pragma unroll
+                for (int r = 0; r < R0; ++r) x[r] = cscale(csub(x[r], cref), a.scale);
             }
             if constexpr (SMEM_IN) __syncthreads();   // the tile is read before the exchange overwrites it
             if (on) {
@@ -835,8 +840,10 @@ template <typename T, int N, int WB_ = 0> struct TpRows {
     static constexpr int PF = tp_pitch(R0), PD = tp_pitch(R1), PP = tp_pitch(RP);
     // exchange elements of one line: forward of N and of 3N/2, backward of N and of 3N/2
     static constexpr int LF = tp_line(R1 * PF), LF2 = tp_line(RP * PF), LD = tp_line(R0 * PD), LP = tp_line(R0 * PP);
-    static constexpr int WB = WB_ ? WB_ : R0 == 8 ? (sizeof(T) == 4 ? 16 : 8) : R0 == 16 ? (sizeof(T) == 4 ? 8 : 4) : R0 == 20 ? 8 : 4;
+    static constexpr int WB = WB_ ? WB_ : R0 == 8 ? (sizeof(T) == 4 ? 16 : 8) : R0 == 16 ? (sizeof(T) == 4 ? 8 : 4) : R0 == 20 ? 8 : R0 == 32 && sizeof(T) == 8 ? 2 : 4;
     static constexpr int NT = R0 * WB;                     // one middle-pass butterfly a thread
+    // (FP64 radix 32 leaves 8 warps: 4 CTAs of 2 lines against 2 of 4 took the multi-output
+    // pass of 512 lines from 2.61 to 2.38 ms and the inverse from 1.34 to 1.26)
     // the inverse's first pass loads: at R0 = 32 its 10..20 butterflies a line are dealt to
     // half as many threads, which then take two middle butterflies each
     static constexpr int PERI = R0 == 32 ? 2 : 1, NTI = NT / PERI;
