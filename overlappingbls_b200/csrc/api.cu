@@ -445,18 +445,21 @@ template <typename T> struct Ops {
             auto ra = rowargs(nullptr, ldx, nullptr, lhx, (long long)ny * L, sc, OP_FWD, nx);
             if ((rc = rows_multi(OP_FWD, nx, ra, m, 3, "press_fwd_rows"))) return rc;
         }
-        // boundary planes H_z(0) and H_z(nz) (:186-200)
-        if (dbot) {
-            auto ra = rowargs(dbot, ldx, Hz, lhx, ny, cst, OP_FWD, nx);
-            if ((rc = rows(OP_FWD, nx, ra, "press_fwd_rows"))) return rc;
+        // boundary planes H_z(0) and H_z(nz) (:186-200); an absent one is zero, and so is its
+        // y-transform
+        const bool top = ctx->opt.top_bc == OBL_TOP_NEUMANN && dtop;
+        if (!dbot && !top) {
+            CK(cudaMemset2DAsync(Hz, sizeof(C2<T>) * S * (L + 1), 0, sizeof(C2<T>) * S, 2, s()));
         } else {
-            CK(cudaMemsetAsync(Hz, 0, sizeof(C2<T>) * S, s()));
-        }
-        if (ctx->opt.top_bc == OBL_TOP_NEUMANN && dtop) {
-            auto ra = rowargs(dtop, ldx, Hz + S * (L + 1), lhx, ny, cst, OP_FWD, nx);
-            if ((rc = rows(OP_FWD, nx, ra, "press_fwd_rows"))) return rc;
-        } else {
-            CK(cudaMemsetAsync(Hz + S * (L + 1), 0, sizeof(C2<T>) * S, s()));
+            for (int zb : {0, L + 1}) {
+                const T *pln = zb ? (top ? dtop : nullptr) : dbot;
+                if (pln) {
+                    auto ra = rowargs(pln, ldx, Hz + S * zb, lhx, ny, cst, OP_FWD, nx);
+                    if ((rc = rows(OP_FWD, nx, ra, "press_fwd_rows"))) return rc;
+                } else {
+                    CK(cudaMemsetAsync(Hz + S * zb, 0, sizeof(C2<T>) * S, s()));
+                }
+            }
         }
         // y c2c (in place), y-Nyquist zeroed
         const bool gf = rhs_ready ? fwd_gform : gform(dpdz_out != nullptr);
@@ -476,9 +479,11 @@ template <typename T> struct Ops {
                               "press_gform_cols")))
                     return rc;
             }
-            auto ca = colargs(Hz, lhx, S, Hz, lhx, S, lhx, 1, 1.0, OP_FWD, ny);
-            ca.zero_nyq = 1;
-            if ((rc = cols(OP_FWD, false, ny, ca, "press_bnd_cols"))) return rc;
+            if (dbot) {
+                auto ca = colargs(Hz, lhx, S, Hz, lhx, S, lhx, 1, 1.0, OP_FWD, ny);
+                ca.zero_nyq = 1;
+                if ((rc = cols(OP_FWD, false, ny, ca, "press_bnd_cols"))) return rc;
+            }
             auto c0 = colargs(Hz + S, lhx, S, Hz + S, lhx, S, 1, L, 1.0, OP_FWD, ny);   // column kx = 0
             c0.zero_nyq = 1;
             if ((rc = cols(OP_FWD, false, ny, c0, "press_mean_cols"))) return rc;
@@ -495,6 +500,7 @@ template <typename T> struct Ops {
             if ((rc = cols(OP_FWD, false, ny, ca, "press_fwd_cols"))) return rc;
         } else {
             for (int zb : {0, L + 1}) {
+                if (!(zb ? top : dbot != nullptr)) continue;
                 auto ca = colargs(Hz + S * zb, lhx, S, Hz + S * zb, lhx, S, lhx, 1, 1.0, OP_FWD, ny);
                 ca.zero_nyq = 1;
                 if ((rc = cols(OP_FWD, false, ny, ca, "press_bnd_cols"))) return rc;
@@ -637,16 +643,18 @@ template <typename T> struct Ops {
             pr.u = (T *)proj->u; pr.v = (T *)proj->v; pr.w = (T *)proj->w;
             pr.npairs = (long long)ny * (L + 1) / 2;
             pr.ldx = ldx; pr.ny = ny; pr.lhx = lhx;
+            const int sf = stress_free < 0 ? (int)ctx->opt.ubc_stress_free : stress_free;
+            pr.L = L; pr.zero_bc = !sf;
             pr.dt_tadv1 = (T)(ctx->dt_nd * kTadv1);
             pr.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD);
             {
                 LaunchScope ls(ctx->rec, "pinv_rows_project", s());
                 if ((rc = chk(PinvLaunch<T>::rows(nx, pr, s()), "pinv_rows_project"))) return rc;
             }
+            if (!sf) return OBL_OK;   // w(1) = w(nz) = 0 were stored by the row pass
             cudaError_t e = cudaSuccess;
             LaunchScope ls(ctx->rec, "project_bc", s());
-            launch_project_bc<T>((T *)proj->u, (T *)proj->v, (T *)proj->w, ldx, ny, ctx->nz,
-                                 stress_free < 0 ? (int)ctx->opt.ubc_stress_free : stress_free, s(), e);
+            launch_project_bc<T>((T *)proj->u, (T *)proj->v, (T *)proj->w, ldx, ny, ctx->nz, sf, s(), e);
             return chk(e, "project_bc");
         }
         // inverse transforms (:231-238): p at 0..L, dpdx/dpdy at 1..L; Hx/Hy/Hz are
@@ -797,10 +805,62 @@ template <typename T> struct Ops {
     int fwd_lines(const obl_step_io *io)
     {
         int rc;
+        if (fwd_batched()) return fwd_batch(io);
         if ((rc = fwd_prepare())) return rc;
         for (int c = 0; c < 4; ++c)
             if ((rc = fwd_field(io, c))) return rc;
         return OBL_OK;
+    }
+    // All four fields in two launches, rows then columns, instead of fifteen, on small grids:
+    // up to 16 MB of x-padded intermediates.  Step times (us, batched / by field): 64x64x64
+    // FP64 (13 MB) 100 / 119, 96x96x64 mixed (15 MB) 130 / 151; 128x128x96 mixed (38 MB)
+    // 276 / 218, 256x256x32 (39 MB) 280 / 238: field by field, the intermediate and the field
+    // are still in L2 when the column passes read them.
+    static constexpr size_t kFwdBatchBytes = (size_t)16 << 20;
+    bool fwd_batched() const
+    {
+        return !ctx->param_fwd_chunk && 4 * sizeof(T) * (size_t)ctx->nxt2 * ctx->nyt * (ctx->nz + 1) <= kFwdBatchBytes;
+    }
+    int fwd_batch(const obl_step_io *io)
+    {
+        const int nlev = ctx->nz + 1, nx = ctx->nxt, ny = ctx->nyt, nx2 = ctx->nxt2, ny2 = ctx->nyt2, lhx = ctx->lhx;
+        const long long S = ctx->sp(), pl = ctx->plane(), plx = (long long)nx2 * ny, plb = (long long)nx2 * ny2;
+        const size_t sb = sizeof(C2<T>) * (size_t)S * (ctx->nz + 1), xsz = (size_t)plx * nlev;
+        int rc;
+        for (int i = 0; i < 5; ++i)
+            if ((rc = ensure(ctx, ctx->spec[i], sb))) return rc;
+        if ((rc = ensure(ctx, ctx->tmp, sizeof(T) * xsz * 4))) return rc;
+        T *xb = (T *)ctx->tmp.p;
+        const T *f[4] = {(const T *)io->u, (const T *)io->v, (const T *)io->w, (const T *)io->theta};
+        RowsFwd3Args<T> ra{};
+        ra.npairs = (long long)ny * nlev / 2; ra.ldx = ctx->ldx; ra.ny = ny; ra.L = ctx->L; ra.z0 = 0;
+        ra.sc_press = ((1.0 / ((double)nx * ny)) / kTadv1) * (1.0 / ctx->dt_nd);
+        ra.kx = ctx->d_kx;
+        ra.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD); ra.twB = twt<T>(ctx, nx, ROLE_TP + ROLE_BWD);
+        ra.twPB = twt<T>(ctx, nx, ROLE_TP + ROLE_PADBWD);
+        RowsFwd3Fields<T> m{};
+        ColsFwdArgs<T> ca{};
+        ca.pad = colargs(nullptr, nx2, plx, nullptr, nx2, plb, nx2, nlev, 1.0 / ny, OP_PAD, ny);
+        ca.ddy = colargs(nullptr, ctx->ldx, pl, nullptr, ctx->ldx, pl, nx, nlev, 1.0 / ny, OP_DERIV, ny);
+        ca.fwd = colargs(nullptr, lhx, S, nullptr, lhx, S, lhx, ctx->L, 1.0, OP_FWD, ny);
+        ca.fwd.zero_nyq = 1;
+        ca.nf = 4;
+        for (int c = 0; c < 4; ++c) {
+            C2<T> *H = c < 3 ? (C2<T> *)ctx->spec[c].p : nullptr;
+            m.src[c] = f[c]; m.dfdx[c] = (T *)io->d[2 * c]; m.xpad[c] = xb + c * xsz; m.H[c] = H;
+            ca.mpad.src[c] = m.xpad[c]; ca.mpad.dst[c] = io->big[c];
+            ca.mddy.src[c] = f[c]; ca.mddy.dst[c] = io->d[2 * c + 1];
+            if (H && !(fwd_gform && c != 1)) {   // G form: H_x and H_z are transformed as G in press()
+                ca.mfwd.src[ca.nfwd] = ca.mfwd.dst[ca.nfwd] = H + S;
+                ++ca.nfwd;
+            }
+        }
+        {
+            LaunchScope ls(ctx->rec, "rows_fwd3", s());
+            if ((rc = chk(RowsFwd3Launch<T>::run_multi(nx, ra, m, 4, s()), "rows_fwd3"))) return rc;
+        }
+        LaunchScope ls(ctx->rec, "cols_fwd", s());
+        return chk(ColsFwdLaunch<T>::run(ny, ca, s()), "cols_fwd");
     }
     int fwd_prepare()
     {

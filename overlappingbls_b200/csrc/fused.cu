@@ -123,6 +123,91 @@ template <typename T, int N> static cudaError_t rows3_run_n(const RowsFwd3Args<T
     return cudaGetLastError();
 }
 
+template <typename T, int N>
+static cudaError_t rows3_multi_n(const RowsFwd3Args<T> &a, const RowsFwd3Fields<T> &m, int nf, cudaStream_t s)
+{
+    using G = TpRows<T, N>;
+    static bool inits[kMaxDevices] = {};
+    cudaError_t e = allow_smem(k_tp_rows_fwd3_multi<T, N>, G::smem_fwd3, inits);
+    if (e != cudaSuccess) return e;
+    const long long nb = (a.npairs + G::WB - 1) / G::WB;
+    if (nb < 1) return cudaSuccess;
+    k_tp_rows_fwd3_multi<T, N><<<(unsigned)(nb * nf), G::NT, G::smem_fwd3, s>>>(a, m, (int)nb);
+    return cudaGetLastError();
+}
+
+template <typename T, int N> struct TpColsFwd {
+    using G = TpGeo<T, N, OP_PAD>;   // one middle butterfly a thread in all three
+    static constexpr int NT = TwoPass<N>::R0 * G::WB;
+    static constexpr size_t smem = sizeof(C2<T>) * (size_t)G::WB * TpLine<N, OP_PAD>::ROWS;
+    static_assert(TpLine<N, OP_DERIV>::ROWS <= TpLine<N, OP_PAD>::ROWS && TpLine<N, OP_FWD>::ROWS <= TpLine<N, OP_PAD>::ROWS, "one exchange for all");
+};
+template <typename T, int N>
+__global__ void __launch_bounds__(TpColsFwd<T, N>::NT, TpGeo<T, N, OP_PAD>::minb) k_tp_cols_fwd(ColsFwdArgs<T> a, int npad, int nddy)
+{
+    constexpr int WB = TpGeo<T, N, OP_PAD>::WB, NT = TpColsFwd<T, N>::NT;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    C2<T> *buf = reinterpret_cast<C2<T> *>(smraw);
+    int u = blockIdx.x;
+    auto unit = [&](ColArgs<T> &c, const MultiPtr<T> &m, int nlines, int &bx, int &z) {
+        const int nbx = (nlines + WB - 1) / WB, f = u / (nbx * c.nlev);
+        u -= f * nbx * c.nlev;
+        z = u / nbx;
+        bx = u - z * nbx;
+        c.src = m.src[f];
+        c.dst = m.dst[f];
+    };
+    int bx, z;
+    if (u < npad) {
+        unit(a.pad, a.mpad, a.pad.ncols / 2, bx, z);
+        tp_cols_unit<T, N, OP_PAD, true, NT, WB>(a.pad, bx, z, buf);
+    } else if ((u -= npad) < nddy) {
+        unit(a.ddy, a.mddy, a.ddy.ncols / 2, bx, z);
+        tp_cols_unit<T, N, OP_DERIV, true, NT, WB>(a.ddy, bx, z, buf);
+    } else {
+        u -= nddy;
+        unit(a.fwd, a.mfwd, a.fwd.ncols, bx, z);
+        tp_cols_unit<T, N, OP_FWD, false, NT, WB>(a.fwd, bx, z, buf);
+    }
+}
+
+template <typename T, int N> static cudaError_t cols_fwd_n(const ColsFwdArgs<T> &a, cudaStream_t s)
+{
+    using G = TpColsFwd<T, N>;
+    constexpr int WB = TpGeo<T, N, OP_PAD>::WB;
+    static bool inits[kMaxDevices] = {};
+    cudaError_t e = allow_smem(k_tp_cols_fwd<T, N>, G::smem, inits);
+    if (e != cudaSuccess) return e;
+    auto units = [&](const ColArgs<T> &c, int nlines, int nf) { return (long long)((nlines + WB - 1) / WB) * c.nlev * nf; };
+    const long long npad = units(a.pad, a.pad.ncols / 2, a.nf), nddy = units(a.ddy, a.ddy.ncols / 2, a.nf),
+                    nfwd = units(a.fwd, a.fwd.ncols, a.nfwd);
+    k_tp_cols_fwd<T, N><<<(unsigned)(npad + nddy + nfwd), G::NT, G::smem, s>>>(a, (int)npad, (int)nddy);
+    return cudaGetLastError();
+}
+
+template <typename T> cudaError_t ColsFwdLaunch<T>::run(int n, const ColsFwdArgs<T> &a, cudaStream_t s)
+{
+    switch (n) {
+#define OBL_CASE(N) case N: return cols_fwd_n<T, N>(a, s);
+        OBL_FOR_EACH_N(OBL_CASE)
+#undef OBL_CASE
+    }
+    return cudaErrorNotSupported;
+}
+template struct ColsFwdLaunch<float>;
+template struct ColsFwdLaunch<double>;
+
+template <typename T>
+cudaError_t RowsFwd3Launch<T>::run_multi(int n, const RowsFwd3Args<T> &a, const RowsFwd3Fields<T> &m, int nf, cudaStream_t s)
+{
+    switch (n) {
+#define OBL_CASE(N) case N: return rows3_multi_n<T, N>(a, m, nf, s);
+        OBL_FOR_EACH_N(OBL_CASE)
+#undef OBL_CASE
+    }
+    return cudaErrorNotSupported;
+}
+
 template <typename T> cudaError_t RowsFwd3Launch<T>::run(int n, const RowsFwd3Args<T> &a, cudaStream_t s)
 {
     switch (n) {

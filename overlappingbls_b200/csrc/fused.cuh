@@ -400,8 +400,39 @@ __global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) k_tp_row
     tp_rows_fwd3_unit<T, N>(a, blockIdx.x, reinterpret_cast<C2<T> *>(smraw));
 }
 
+// The same for several fields in one launch: field f's pointers replace src, dfdx, xpad, H.
+template <typename T> struct RowsFwd3Fields {
+    const T *src[4];
+    T *dfdx[4], *xpad[4];
+    C2<T> *H[4];
+};
+template <typename T, int N>
+__global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) k_tp_rows_fwd3_multi(RowsFwd3Args<T> a0, RowsFwd3Fields<T> m, int nb)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int f = blockIdx.x / nb;   // nb CTAs per field
+    RowsFwd3Args<T> a = a0;
+    a.src = m.src[f];
+    a.dfdx = m.dfdx[f];
+    a.xpad = m.xpad[f];
+    a.H = m.H[f];
+    tp_rows_fwd3_unit<T, N>(a, blockIdx.x - f * nb, reinterpret_cast<C2<T> *>(smraw));
+}
+
 template <typename T> struct RowsFwd3Launch {
     static cudaError_t run(int n, const RowsFwd3Args<T> &a, cudaStream_t s);
+    static cudaError_t run_multi(int n, const RowsFwd3Args<T> &a, const RowsFwd3Fields<T> &m, int nf, cudaStream_t s);
+};
+
+// The forward pass's column work of all fields in one launch: units of the y-pad, of ddy and
+// of the RHS y-transform, one after the other in blockIdx.x.
+template <typename T> struct ColsFwdArgs {
+    ColArgs<T> pad, ddy, fwd;
+    MultiPtr<T> mpad, mddy, mfwd;
+    int nf, nfwd;                         // fields; spectra
+};
+template <typename T> struct ColsFwdLaunch {
+    static cudaError_t run(int n, const ColsFwdArgs<T> &a, cudaStream_t s);
 };
 
 // ----------------------------------------------------------------------------- fused inverse
@@ -518,6 +549,7 @@ template <typename T> struct PinvRowArgs {
     const C2<T> *twF;                     // two-pass table of nx
     int w_from_1;                         // 0: w updated from level 2 (bottom rank, jz_min = 2);
                                           // 1: from level 1 (the z-slab of a rank above it)
+    int L, zero_bc;                       // zero_bc: also w(1) = w(nz) = 0 (110_project.f90:55-60), nz = L+1
 };
 
 // Unit: component q (0: p; 1: dpdx and u; 2: dpdy and v; 3: dpdz and w) of the WB row pairs
@@ -556,7 +588,7 @@ __device__ __forceinline__ void tp_pinv_rows_unit(const PinvRowArgs<T> &a, int q
         }
     };
     T fa[R1], fb[R1];
-    T *f = nullptr, *out = nullptr;
+    T *f = nullptr, *out = nullptr, *bc = nullptr;
     bool act = false, proj = false;
     // the rows of the field to update are on their way while the exchange is read
     auto pre = [&](int ln, int j) {
@@ -567,6 +599,7 @@ __device__ __forceinline__ void tp_pinv_rows_unit(const PinvRowArgs<T> &a, int q
         proj = act && (q == 1 || q == 2 || (q == 3 && z >= (a.w_from_1 ? 1 : 2)));   // jz_min for w
         f = (q == 1 ? a.u : q == 2 ? a.v : a.w) + pl * z + off;
         out = q == 0 ? a.p + pl * z + off : (q == 1 ? a.dpdx : q == 2 ? a.dpdy : a.dpdz) + pl * (z - 1) + off;
+        bc = act && q == 3 && a.zero_bc && (z == 1 || z == a.L) ? a.w + pl * (z == 1 ? 1 : z + 1) + off : nullptr;
 #pragma unroll
         for (int r = 0; r < R1; ++r) {
             fa[r] = proj ? f[r * R0] : (T)0;
@@ -584,8 +617,13 @@ __device__ __forceinline__ void tp_pinv_rows_unit(const PinvRowArgs<T> &a, int q
             asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
         }
     }
-    tp_rows_inv<T, N, WB_>(src, op, buf, a.twF, pre, [&](int, int, const C(&x)[R1]) {
+    tp_rows_inv<T, N, WB_>(src, op, buf, a.twF, pre, [&](int, int j, const C(&x)[R1]) {
         if (!act) return;
+        if (bc) {   // whole rows, pads included
+#pragma unroll
+            for (int r = 0; r < R1; ++r) bc[r * R0] = bc[a.ldx + r * R0] = (T)0;
+            if (j < 2) bc[N] = bc[a.ldx + N] = (T)0;
+        }
 #pragma unroll
         for (int r = 0; r < R1; ++r) {
             out[r * R0] = x[r].x;
