@@ -462,7 +462,7 @@ template <typename T> struct Ops {
             }
         }
         // y c2c (in place), y-Nyquist zeroed
-        const bool gf = rhs_ready ? fwd_gform : gform(dpdz_out != nullptr);
+        const bool gf = rhs_ready ? fwd_gform : gform();
         if (gf) {
             // H_y as it is; G = i*kx*H_x + (H_z(z+1) - H_z(z) [+ H_z(0)])/dz formed from the
             // x-spectra and transformed over H_x; H_z at level 0, and at levels 1..L only in
@@ -514,7 +514,7 @@ template <typename T> struct Ops {
         ta.dph = dpdz_out ? (C2<T> *)ctx->spec[4].p : nullptr;
         ta.neumann_top = ctx->opt.top_bc == OBL_TOP_NEUMANN;
         ta.gform = gf ? 1 : 0;
-        const int P = solve_parts(ta.dph != nullptr);
+        const int P = solve_parts();
         if (P > 1) {
             // the columns split into segments solved at once (partitioned Thomas, as across
             // z-ranks), then the reduced interface system and the back substitution
@@ -625,48 +625,41 @@ template <typename T> struct Ops {
                 if (e != cudaSuccess) return cuda_fail(ctx, e, "tdma");
             }
         }
-        if (proj && dpdz_out) {
-            // fused inverse + project: one y-inverse pass over p_hat and the dpdz spectrum,
-            // one x-inverse pass over the rows that also applies project()
-            PinvColArgs<T> pc{};
-            pc.ph = ph; pc.dph = (const C2<T> *)ctx->spec[4].p;
-            pc.Xp = Hz; pc.Xdy = Hy; pc.Xdz = (C2<T> *)ctx->spec[4].p;
-            pc.S = S; pc.lhx = lhx; pc.kx = ctx->d_kx; pc.ky = ctx->d_ky2;
-            pc.twB = twt<T>(ctx, ny, ROLE_TP + ROLE_BWD);
-            {
-                LaunchScope ls(ctx->rec, "pinv_cols", s());
-                if ((rc = chk(PinvLaunch<T>::cols(ny, pc, L + 1, s()), "pinv_cols"))) return rc;
-            }
-            PinvRowArgs<T> pr{};
-            pr.Xp = Hz; pr.kx = ctx->d_kx; pr.Xdy = Hy; pr.Xdz = (const C2<T> *)ctx->spec[4].p;
-            pr.p = p; pr.dpdx = dpdx; pr.dpdy = dpdy; pr.dpdz = dpdz_out;
+        // inverse transforms (:231-238), p at 0..L, dpdx/dpdy (and the spectral dpdz) at 1..L:
+        // one y-inverse pass over p_hat (and the dpdz spectrum), one x-inverse pass over the
+        // rows that also applies project() when asked for.  dpdx takes its y-inverse from p's
+        // (i*kx commutes with it): two y-transforms instead of three for p, dpdx, dpdy
+        PinvColArgs<T> pc{};
+        pc.ph = ph; pc.dph = dpdz_out ? (const C2<T> *)ctx->spec[4].p : nullptr;
+        pc.Xp = Hz; pc.Xdy = Hy; pc.Xdz = dpdz_out ? (C2<T> *)ctx->spec[4].p : nullptr;
+        pc.S = S; pc.lhx = lhx; pc.kx = ctx->d_kx; pc.ky = ctx->d_ky2;
+        pc.twB = twt<T>(ctx, ny, ROLE_TP + ROLE_BWD);
+        {
+            LaunchScope ls(ctx->rec, "pinv_cols", s());
+            if ((rc = chk(PinvLaunch<T>::cols(ny, pc, L + 1, s()), "pinv_cols"))) return rc;
+        }
+        PinvRowArgs<T> pr{};
+        pr.Xp = Hz; pr.kx = ctx->d_kx; pr.Xdy = Hy; pr.Xdz = pc.Xdz;
+        pr.p = p; pr.dpdx = dpdx; pr.dpdy = dpdy; pr.dpdz = dpdz_out;
+        if (proj) {
             pr.u = (T *)proj->u; pr.v = (T *)proj->v; pr.w = (T *)proj->w;
-            pr.npairs = (long long)ny * (L + 1) / 2;
-            pr.ldx = ldx; pr.ny = ny; pr.lhx = lhx;
-            const int sf = stress_free < 0 ? (int)ctx->opt.ubc_stress_free : stress_free;
-            pr.L = L; pr.zero_bc = !sf;
-            pr.dt_tadv1 = (T)(ctx->dt_nd * kTadv1);
-            pr.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD);
-            {
-                LaunchScope ls(ctx->rec, "pinv_rows_project", s());
-                if ((rc = chk(PinvLaunch<T>::rows(nx, pr, s()), "pinv_rows_project"))) return rc;
-            }
-            if (!sf) return OBL_OK;   // w(1) = w(nz) = 0 were stored by the row pass
-            cudaError_t e = cudaSuccess;
-            LaunchScope ls(ctx->rec, "project_bc", s());
-            launch_project_bc<T>((T *)proj->u, (T *)proj->v, (T *)proj->w, ldx, ny, ctx->nz, sf, s(), e);
-            return chk(e, "project_bc");
         }
-        // inverse transforms (:231-238): p at 0..L, dpdx/dpdy at 1..L; Hx/Hy/Hz are
-        // free now and hold the y-inverses
-        if ((rc = ifftn(ph, Hz, p, 0, L + 1, 0))) return rc;
-        if ((rc = ifftn(ph + S, Hx, dpdx, 0, L, 1))) return rc;
-        if ((rc = ifftn(ph + S, Hy, dpdy, 0, L, 2))) return rc;
-        if (dpdz_out) {
-            C2<T> *dph = (C2<T> *)ctx->spec[4].p + S;
-            if ((rc = ifftn(dph, dph, dpdz_out, 0, L, 0))) return rc;
+        pr.npairs = (long long)ny * (L + 1) / 2;
+        pr.ldx = ldx; pr.ny = ny; pr.lhx = lhx;
+        const int sf = stress_free < 0 ? (int)ctx->opt.ubc_stress_free : stress_free;
+        pr.L = L; pr.zero_bc = proj && !sf;
+        pr.dt_tadv1 = (T)(ctx->dt_nd * kTadv1);
+        pr.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD);
+        {
+            const char *name = proj ? "pinv_rows_project" : "pinv_rows";
+            LaunchScope ls(ctx->rec, name, s());
+            if ((rc = chk(PinvLaunch<T>::rows(nx, pr, s()), name))) return rc;
         }
-        return OBL_OK;
+        if (!proj || !sf) return OBL_OK;   // w(1) = w(nz) = 0 were stored by the row pass
+        cudaError_t e = cudaSuccess;
+        LaunchScope ls(ctx->rec, "project_bc", s());
+        launch_project_bc<T>((T *)proj->u, (T *)proj->v, (T *)proj->w, ldx, ny, ctx->nz, sf, s(), e);
+        return chk(e, "project_bc");
     }
 
     int dpdz(const T *p, T *dp)
@@ -924,7 +917,7 @@ template <typename T> struct Ops {
         // param "fused": 0 multi-output line kernels (default), 1 cluster-fused forward pass,
         // 2 the plain composition of the per-routine entry points
         if (ctx->param_fused == 0 || (ctx->param_fused == 1 && ctx->nxt == ctx->nyt)) {
-            fwd_gform = ctx->param_fused == 0 && gform(true);
+            fwd_gform = ctx->param_fused == 0 && gform();
             if ((rc = ctx->param_fused == 0 ? fwd_lines(io) : fwd_fused(io))) return rc;
             return press(f[0], f[1], f[2], (const T *)io->divtz_bot, (const T *)io->divtz_top, (T *)io->p,
                          (T *)io->dp[0], (T *)io->dp[1], (T *)io->dp[2], true, io);
@@ -1177,23 +1170,20 @@ template <typename T> struct Ops {
     // the Neumann-top step with spectral dpdz and the three-spectra RHS.
     int isl_parts(const TdmaArgs<T> &ta) const
     {
-        if (!ctx->n_isl || ta.gform || !ta.dph || ctx->opt.top_bc != OBL_TOP_NEUMANN) return 1;
+        if (!ctx->n_isl || ta.gform || ctx->opt.top_bc != OBL_TOP_NEUMANN) return 1;
         const long long P = ctx->param_isl_segments > 0 ? ctx->param_isl_segments : 16;
         const long long cap = std::min<long long>(kSlabMaxRanks, ctx->L / 8);
         return (int)std::max<long long>(1, std::min<long long>(P, cap));
     }
-    int solve_parts(bool dpdz) const
-    {
-        return (ctx->opt.top_bc == OBL_TOP_NEUMANN && dpdz) ? seg_parts(ctx->sp(), ctx->L) : 1;
-    }
+    int solve_parts() const { return ctx->opt.top_bc == OBL_TOP_NEUMANN ? seg_parts(ctx->sp(), ctx->L) : 1; }
     // the RHS in G form: the one-sweep and register-segmented solves take it; the
     // column-segmented solve keeps the three transformed spectra.  By default only with
     // FP64 storage: the RHS is a divergence whose terms nearly cancel, and G's partial sum
     // rounded to FP32 before the transform costs the FP64 island columns their exact RHS
     // assembly (at 512^2 x 256 the mixed form's p error rose from 1.4e-7 to 8.5e-6).
-    bool gform(bool dpdz) const
+    bool gform() const
     {
-        return (ctx->param_gform == 2 || (ctx->param_gform == 1 && ctx->f64)) && solve_parts(dpdz) == 1;
+        return (ctx->param_gform == 2 || (ctx->param_gform == 1 && ctx->f64)) && solve_parts() == 1;
     }
     // set by the step before its line-kernel forward pass: fwd_field leaves H_x and H_z to
     // press(); the z-slab path, which transforms all three, keeps it false
@@ -2348,7 +2338,7 @@ template <typename HT, typename T> static int step_host_overlapped(obl_ctx *ctx,
         CK(cudaEventRecord(ctx->ev[c], ci));
     }
     Ops<T> o{ctx};
-    o.fwd_gform = o.gform(true);
+    o.fwd_gform = o.gform();
     if ((rc = o.fwd_prepare())) return rc;
     for (int c = 0; c < 4; ++c) {
         CK(cudaStreamWaitEvent(s, ctx->ev[c], 0));

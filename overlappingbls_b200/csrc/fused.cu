@@ -228,7 +228,7 @@ template <typename T, int N> static cudaError_t pinv_cols_n(const PinvColArgs<T>
     cudaError_t e = allow_smem(k_tp_cols_pinv<T, N>, G::smem, inits);
     if (e != cudaSuccess) return e;
     const int nbx = (a.lhx + G::WB - 1) / G::WB;
-    dim3 grid(nbx + (nbx + 1) / 2, nlev);
+    dim3 grid(a.dph ? nbx + (nbx + 1) / 2 : nbx, nlev);
     k_tp_cols_pinv<T, N><<<grid, G::NT, G::smem, s>>>(a);
     return cudaGetLastError();
 }
@@ -240,7 +240,7 @@ template <typename T, int N> static cudaError_t pinv_rows_n(const PinvRowArgs<T>
     constexpr size_t sm = sizeof(C2<T>) * (size_t)G::WB * G::LF;
     cudaError_t e = allow_smem(k_tp_rows_pinv<T, N>, sm, inits);
     if (e != cudaSuccess) return e;
-    const long long grid = 4 * ((a.npairs + G::WB - 1) / G::WB);
+    const long long grid = (a.dpdz ? 4 : 3) * ((a.npairs + G::WB - 1) / G::WB);
     if (grid < 1) return cudaSuccess;
     k_tp_rows_pinv<T, N><<<(unsigned)grid, G::NTI, sm, s>>>(a);
     return cudaGetLastError();

@@ -475,7 +475,7 @@ __device__ __forceinline__ void tp_pinv_cols_unit(const PinvColArgs<T> &a, int u
     const bool pp = u < nbx;                        // p_hat's unit
     if (!pp && z == 0) return;                      // level 0 needs p only
     const int g0 = pp ? u : 2 * (u - nbx), g1 = pp ? u : g0 + 1;
-    const int nt = pp ? (z == 0 ? 1 : 2) : (g1 < nbx ? 2 : 1);
+    const int nt = pp ? (z == 0 ? 1 : 2) : (g1 < nbx ? 2 : 1);   // (p_hat alone: a grid of nbx units)
     auto load = [&](const C *src, int g, C(&v)[R1]) {
         const int gl = g * WB + line;
 #pragma unroll
@@ -541,8 +541,8 @@ template <typename T, int N> __global__ void __launch_bounds__(TpPinv<T, N>::NT,
 template <typename T> struct PinvRowArgs {
     const C2<T> *Xp, *Xdy, *Xdz;          // (lhx, ny, 0..L); dpdx's is i*kx*Xp
     const double *kx;                     // kx(lhx), Nyquist entry 0
-    T *p, *dpdx, *dpdy, *dpdz;            // p (ldx, ny, 0:nz); d* (ldx, ny, 1:nz)
-    T *u, *v, *w;                         // updated in place (ldx, ny, 0:nz)
+    T *p, *dpdx, *dpdy, *dpdz;            // p (ldx, ny, 0:nz); d* (ldx, ny, 1:nz); dpdz optional
+    T *u, *v, *w;                         // updated in place (ldx, ny, 0:nz); u = nullptr: no project()
     long long npairs;                     // ny*(L+1)/2
     int ldx, ny, lhx;
     T dt_tadv1;                           // dt*tadv1
@@ -596,7 +596,7 @@ __device__ __forceinline__ void tp_pinv_rows_unit(const PinvRowArgs<T> &a, int q
         const long long r0 = row0(act ? ln : 0);
         const int z = (int)(r0 / a.ny);
         const long long off = (r0 % a.ny) * a.ldx + j;
-        proj = act && (q == 1 || q == 2 || (q == 3 && z >= (a.w_from_1 ? 1 : 2)));   // jz_min for w
+        proj = act && a.u && (q == 1 || q == 2 || (q == 3 && z >= (a.w_from_1 ? 1 : 2)));   // jz_min for w
         f = (q == 1 ? a.u : q == 2 ? a.v : a.w) + pl * z + off;
         out = q == 0 ? a.p + pl * z + off : (q == 1 ? a.dpdx : q == 2 ? a.dpdy : a.dpdz) + pl * (z - 1) + off;
         bc = act && q == 3 && a.zero_bc && (z == 1 || z == a.L) ? a.w + pl * (z == 1 ? 1 : z + 1) + off : nullptr;
@@ -607,7 +607,7 @@ __device__ __forceinline__ void tp_pinv_rows_unit(const PinvRowArgs<T> &a, int q
         }
     };
     // the update's rows into L2 before the first pass: one 128-byte line per lane
-    if (q > 0) {
+    if (q > 0 && a.u) {
         constexpr int EL = 128 / sizeof(T), PL = (N + EL - 1) / EL;
         for (int i = threadIdx.x; i < 2 * PL * G::WB; i += G::NTI) {
             const int ln = i / (2 * PL);
@@ -640,7 +640,8 @@ template <typename T, int N>
 __global__ void __launch_bounds__(TpRows<T, N>::NTI, TpRows<T, N>::minbI) k_tp_rows_pinv(PinvRowArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    tp_pinv_rows_unit<T, N>(a, blockIdx.x & 3, (long long)(blockIdx.x >> 2) * TpRows<T, N>::WB, reinterpret_cast<C2<T> *>(smraw));
+    const unsigned nq = a.dpdz ? 4 : 3;
+    tp_pinv_rows_unit<T, N>(a, (int)(blockIdx.x % nq), (long long)(blockIdx.x / nq) * TpRows<T, N>::WB, reinterpret_cast<C2<T> *>(smraw));
 }
 
 template <typename T> struct PinvLaunch {

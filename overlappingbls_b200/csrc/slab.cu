@@ -218,7 +218,7 @@ __device__ __forceinline__ void slab_rows_out(const SlabArgs<T> &a, long long q,
     slab_down<T, TC, ISLAND>(R, L, [&](int j, TC c, CC y, TC v) {
         const CC x = mk<TC>(y.x - v * xb.x - c * xn.x, y.y - v * xb.y - c * xn.y);
         ph[S * j] = mk<T>((T)x.x, (T)x.y);
-        dph[S * (j + 1)] = mk<T>((T)((xn.x - x.x) * rdz), (T)((xn.y - x.y) * rdz));
+        if (a.dph) dph[S * (j + 1)] = mk<T>((T)((xn.x - x.x) * rdz), (T)((xn.y - x.y) * rdz));
         xn = x;
     });
     // p_hat(0): the last unknown of the rank below, or on rank 0 the Neumann ghost
@@ -230,7 +230,7 @@ __device__ __forceinline__ void slab_rows_out(const SlabArgs<T> &a, long long q,
         x0 = mk<TC>(xn.x - dz * (TC)h.x, xn.y - dz * (TC)h.y);
     }
     if (a.own_p0) ph[0] = mk<T>((T)x0.x, (T)x0.y);
-    dph[S] = mk<T>((T)((xn.x - x0.x) * rdz), (T)((xn.y - x0.y) * rdz));
+    if (a.dph) dph[S] = mk<T>((T)((xn.x - x0.x) * rdz), (T)((xn.y - x0.y) * rdz));
 }
 
 // The reduced interface system and the rank's rows of one column; t as in slab_column.
@@ -245,7 +245,8 @@ __device__ __forceinline__ void slab_finish_column(const SlabArgs<T> &a, long lo
     C2<T> *ph = a.phat + q, *dph = a.dph + q;
     if (ix == a.lhx - 1 || iy == a.nyt / 2) {
         for (int z = a.own_p0 ? 0 : 1; z <= L; ++z) ph[S * z] = mk<T>(0, 0);
-        for (int z = 1; z <= L; ++z) dph[S * z] = mk<T>(0, 0);
+        if (a.dph)
+            for (int z = 1; z <= L; ++z) dph[S * z] = mk<T>(0, 0);
         return;
     }
     // interface unknowns X_k = (first_k, last_k):  X_k + A_k X_{k-1} + C_k X_{k+1} = Y_k,
@@ -328,7 +329,7 @@ template <typename T> __device__ __forceinline__ SlabArgs<T> seg_view(const Slab
     b.Hy = a.Hy + off;
     b.Hz = a.Hz + off;
     b.phat = a.phat + off;
-    b.dph = a.dph + off;
+    b.dph = a.dph ? a.dph + off : nullptr;
     b.v = a.v + off;
     b.cp = a.cp + off;
     b.iy = a.iy + ioff;
