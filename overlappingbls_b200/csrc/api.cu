@@ -1150,19 +1150,25 @@ template <typename T> struct Ops {
         a.own_p0 = 1;
         return a;
     }
-    // Segments of the single-domain column solve: enough (kx,ky)-column segments to fill
-    // the GPU (8 resident blocks of 128 threads per SM) when the columns alone do not, at
-    // least 8 levels each; 1 = the sequential sweep.
+    // Segments of the single-domain column solve (1 = whole columns).  FP32 storage: the
+    // register-segmented solve has no scratch round trip and wins from 16384 columns on
+    // (solve and RHS transforms, us, segments / whole: 192x192x128 137 / 132, 256x256x128
+    // 203 / 172, 256x256x256 374 / 282; below, 128x128x128 88 / 103).  FP64 sweeps whole
+    // columns from 49152 on (320x240x65: 263 / 225; 256x256x256 483 / 578).  Else enough
+    // segments to fill the GPU (8 resident blocks of 128 threads per SM), at least 8 levels
+    // each, a power of two (equal segments: 256x256x128 FP64 273 with 4, 307 with 5).
     int seg_parts(long long S, int L) const
     {
         if (ctx->param_tdma_segments > 0) return (int)std::min<long long>(ctx->param_tdma_segments, L);
-        if (S >= 65536) return 1;
+        if (S >= (!ctx->f64 && ctx->param_tdma_reg && tdma_reg_supported(L) ? 16384 : 49152)) return 1;
         int dev = 0, nsm = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         const long long want = ((long long)nsm * 8 * 128 + S - 1) / S;
-        const long long P = std::min<long long>(std::min<long long>(want, kSlabMaxRanks), L / 8);
-        return P > 1 ? (int)P : 1;
+        const long long most = std::min<long long>(std::min<long long>(want, kSlabMaxRanks), L / 8);
+        int P = 1;
+        while (2 * P <= most) P *= 2;
+        return P;
     }
     // the solve's column segments for this context (with the spectral dpdz or without)
     // Segments of each FP64 island column in the mixed mode's whole-column solves (1 = the
