@@ -804,12 +804,14 @@ template <typename T> struct Ops {
             if ((rc = fwd_field(io, c))) return rc;
         return OBL_OK;
     }
-    // All four fields in two launches, rows then columns, instead of fifteen, on small grids:
-    // up to 16 MB of x-padded intermediates.  Step times (us, batched / by field): 64x64x64
-    // FP64 (13 MB) 100 / 119, 96x96x64 mixed (15 MB) 130 / 151; 128x128x96 mixed (38 MB)
-    // 276 / 218, 256x256x32 (39 MB) 280 / 238: field by field, the intermediate and the field
-    // are still in L2 when the column passes read them.
-    static constexpr size_t kFwdBatchBytes = (size_t)16 << 20;
+    // All four fields in two launches, rows then columns, instead of fifteen: up to 512 MB of
+    // x-padded intermediates.  Fewer partial last waves, and the column passes of every field
+    // and kind fill one another's gaps.  Step times (us, batched / field by field): 64x64x64
+    // FP64 (13 MB) 71 / 119, 128x128x96 mixed (38 MB) 161 / 218, 256x256x128 (204 MB) 597 /
+    // 692, 512x512x64 (415 MB) 1180 / 1272, 384x384x128 (460 MB) 1308 / 1363; beyond, one
+    // field's launch fills the GPU and its y-pad has the tensor copies: 512x512x256 (1.6 GB)
+    // 4693 / 4630, FP64 10235 / 10001.
+    static constexpr size_t kFwdBatchBytes = (size_t)512 << 20;
     bool fwd_batched() const
     {
         return !ctx->param_fwd_chunk && 4 * sizeof(T) * (size_t)ctx->nxt2 * ctx->nyt * (ctx->nz + 1) <= kFwdBatchBytes;

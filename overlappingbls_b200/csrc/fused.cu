@@ -143,32 +143,25 @@ template <typename T, int N> struct TpColsFwd {
     static_assert(TpLine<N, OP_DERIV>::ROWS <= TpLine<N, OP_PAD>::ROWS && TpLine<N, OP_FWD>::ROWS <= TpLine<N, OP_PAD>::ROWS, "one exchange for all");
 };
 template <typename T, int N>
-__global__ void __launch_bounds__(TpColsFwd<T, N>::NT, TpGeo<T, N, OP_PAD>::minb) k_tp_cols_fwd(ColsFwdArgs<T> a, int npad, int nddy)
+__global__ void __launch_bounds__(TpColsFwd<T, N>::NT, TpGeo<T, N, OP_PAD>::minb)
+    k_tp_cols_fwd(const __grid_constant__ ColsFwdArgs<T> a, int npad, int nddy)
 {
     constexpr int WB = TpGeo<T, N, OP_PAD>::WB, NT = TpColsFwd<T, N>::NT;
     extern __shared__ __align__(128) unsigned char smraw[];
     C2<T> *buf = reinterpret_cast<C2<T> *>(smraw);
-    int u = blockIdx.x;
-    auto unit = [&](ColArgs<T> &c, const MultiPtr<T> &m, int nlines, int &bx, int &z) {
-        const int nbx = (nlines + WB - 1) / WB, f = u / (nbx * c.nlev);
-        u -= f * nbx * c.nlev;
-        z = u / nbx;
-        bx = u - z * nbx;
+    // unit u of one of the three lists: field, plane, line group
+    auto run = [&](auto op, const ColArgs<T> &c0, const MultiPtr<T> &m, int nlines, int u) {
+        constexpr int OP = decltype(op)::value;
+        const int nbx = (nlines + WB - 1) / WB, f = u / (nbx * c0.nlev), v = u - f * nbx * c0.nlev, z = v / nbx;
+        ColArgs<T> c = c0;
         c.src = m.src[f];
         c.dst = m.dst[f];
+        tp_cols_unit<T, N, OP, OP != OP_FWD, NT, WB>(c, v - z * nbx, z, buf);
     };
-    int bx, z;
-    if (u < npad) {
-        unit(a.pad, a.mpad, a.pad.ncols / 2, bx, z);
-        tp_cols_unit<T, N, OP_PAD, true, NT, WB>(a.pad, bx, z, buf);
-    } else if ((u -= npad) < nddy) {
-        unit(a.ddy, a.mddy, a.ddy.ncols / 2, bx, z);
-        tp_cols_unit<T, N, OP_DERIV, true, NT, WB>(a.ddy, bx, z, buf);
-    } else {
-        u -= nddy;
-        unit(a.fwd, a.mfwd, a.fwd.ncols, bx, z);
-        tp_cols_unit<T, N, OP_FWD, false, NT, WB>(a.fwd, bx, z, buf);
-    }
+    const int u = blockIdx.x;
+    if (u < npad) run(std::integral_constant<int, OP_PAD>{}, a.pad, a.mpad, a.pad.ncols / 2, u);
+    else if (u < npad + nddy) run(std::integral_constant<int, OP_DERIV>{}, a.ddy, a.mddy, a.ddy.ncols / 2, u - npad);
+    else run(std::integral_constant<int, OP_FWD>{}, a.fwd, a.mfwd, a.fwd.ncols, u - npad - nddy);
 }
 
 template <typename T, int N> static cudaError_t cols_fwd_n(const ColsFwdArgs<T> &a, cudaStream_t s)

@@ -401,13 +401,16 @@ __global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) k_tp_row
 }
 
 // The same for several fields in one launch: field f's pointers replace src, dfdx, xpad, H.
+// (__grid_constant__: indexing the by-value argument made every thread copy it to local
+// memory first)
 template <typename T> struct RowsFwd3Fields {
     const T *src[4];
     T *dfdx[4], *xpad[4];
     C2<T> *H[4];
 };
 template <typename T, int N>
-__global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) k_tp_rows_fwd3_multi(RowsFwd3Args<T> a0, RowsFwd3Fields<T> m, int nb)
+__global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) 
+    k_tp_rows_fwd3_multi(const __grid_constant__ RowsFwd3Args<T> a0, const __grid_constant__ RowsFwd3Fields<T> m, int nb)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int f = blockIdx.x / nb;   // nb CTAs per field

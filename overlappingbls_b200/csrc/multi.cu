@@ -6,7 +6,8 @@
 namespace obl {
 
 template <typename T, int N, int OP>
-__global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) k_tp_rows_multi(RowArgs<T> a0, MultiPtr<T> m, int nb)
+__global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) 
+    k_tp_rows_multi(RowArgs<T> a0, const __grid_constant__ MultiPtr<T> m, int nb)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int f = blockIdx.x / nb;   // nb CTAs per field
@@ -17,7 +18,8 @@ __global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb) k_tp_row
 }
 
 template <typename T, int N, int OP, bool REAL>
-__global__ void __launch_bounds__(TpGeo<T, N, OP>::NT, TpGeo<T, N, OP>::minb) k_tp_cols_multi(ColArgs<T> a0, MultiPtr<T> m)
+__global__ void __launch_bounds__(TpGeo<T, N, OP>::NT, TpGeo<T, N, OP>::minb) 
+    k_tp_cols_multi(ColArgs<T> a0, const __grid_constant__ MultiPtr<T> m)
 {
     using G = TpGeo<T, N, OP>;
     extern __shared__ __align__(128) unsigned char smraw[];
