@@ -462,7 +462,7 @@ template <typename T> struct Ops {
             }
         }
         // y c2c (in place), y-Nyquist zeroed
-        const bool gf = rhs_ready ? fwd_gform : gform();
+        const bool gf = rhs_ready ? fwd_gform : gform(dpdz_out != nullptr);
         if (gf) {
             // H_y as it is; G = i*kx*H_x + (H_z(z+1) - H_z(z) [+ H_z(0)])/dz formed from the
             // x-spectra and transformed over H_x; H_z at level 0, and at levels 1..L only in
@@ -514,7 +514,7 @@ template <typename T> struct Ops {
         ta.dph = dpdz_out ? (C2<T> *)ctx->spec[4].p : nullptr;
         ta.neumann_top = ctx->opt.top_bc == OBL_TOP_NEUMANN;
         ta.gform = gf ? 1 : 0;
-        const int P = solve_parts();
+        const int P = solve_parts(ta.dph != nullptr);
         if (P > 1) {
             // the columns split into segments solved at once (partitioned Thomas, as across
             // z-ranks), then the reduced interface system and the back substitution
@@ -919,7 +919,7 @@ template <typename T> struct Ops {
         // param "fused": 0 multi-output line kernels (default), 1 cluster-fused forward pass,
         // 2 the plain composition of the per-routine entry points
         if (ctx->param_fused == 0 || (ctx->param_fused == 1 && ctx->nxt == ctx->nyt)) {
-            fwd_gform = ctx->param_fused == 0 && gform();
+            fwd_gform = ctx->param_fused == 0 && gform(true);
             if ((rc = ctx->param_fused == 0 ? fwd_lines(io) : fwd_fused(io))) return rc;
             return press(f[0], f[1], f[2], (const T *)io->divtz_bot, (const T *)io->divtz_top, (T *)io->p,
                          (T *)io->dp[0], (T *)io->dp[1], (T *)io->dp[2], true, io);
@@ -1183,15 +1183,20 @@ template <typename T> struct Ops {
         const long long cap = std::min<long long>(kSlabMaxRanks, ctx->L / 8);
         return (int)std::max<long long>(1, std::min<long long>(P, cap));
     }
-    int solve_parts() const { return ctx->opt.top_bc == OBL_TOP_NEUMANN ? seg_parts(ctx->sp(), ctx->L) : 1; }
+    // (with the spectral dpdz or without: press_stag_array alone keeps whole columns, whose
+    // FP64 error is the smaller, 2e-14 against 1.6e-13 in p at 192x192x128)
+    int solve_parts(bool dpdz) const
+    {
+        return (ctx->opt.top_bc == OBL_TOP_NEUMANN && dpdz) ? seg_parts(ctx->sp(), ctx->L) : 1;
+    }
     // the RHS in G form: the one-sweep and register-segmented solves take it; the
     // column-segmented solve keeps the three transformed spectra.  By default only with
     // FP64 storage: the RHS is a divergence whose terms nearly cancel, and G's partial sum
     // rounded to FP32 before the transform costs the FP64 island columns their exact RHS
     // assembly (at 512^2 x 256 the mixed form's p error rose from 1.4e-7 to 8.5e-6).
-    bool gform() const
+    bool gform(bool dpdz) const
     {
-        return (ctx->param_gform == 2 || (ctx->param_gform == 1 && ctx->f64)) && solve_parts() == 1;
+        return (ctx->param_gform == 2 || (ctx->param_gform == 1 && ctx->f64)) && solve_parts(dpdz) == 1;
     }
     // set by the step before its line-kernel forward pass: fwd_field leaves H_x and H_z to
     // press(); the z-slab path, which transforms all three, keeps it false
@@ -2346,7 +2351,7 @@ template <typename HT, typename T> static int step_host_overlapped(obl_ctx *ctx,
         CK(cudaEventRecord(ctx->ev[c], ci));
     }
     Ops<T> o{ctx};
-    o.fwd_gform = o.gform();
+    o.fwd_gform = o.gform(true);
     if ((rc = o.fwd_prepare())) return rc;
     for (int c = 0; c < 4; ++c) {
         CK(cudaStreamWaitEvent(s, ctx->ev[c], 0));
