@@ -216,12 +216,12 @@ template <typename T> struct Ops {
     }
 
     // plan twiddle tables of the forward / backward transform of a line op of base length n
-    void tables(int op, int n, const C2<T> *&f, const C2<T> *&b, int family)
+    void tables(int op, int n, const C2<T> *&f, const C2<T> *&b)
     {
         const int rf = op == OP_UNPAD ? ROLE_PADFWD : ROLE_FWD;
         const int rb = op == OP_PAD ? ROLE_PADBWD : ROLE_BWD;
-        f = twt<T>(ctx, n, family + rf);
-        b = twt<T>(ctx, n, family + rb);
+        f = twt<T>(ctx, n, ROLE_TP + rf);
+        b = twt<T>(ctx, n, ROLE_TP + rb);
     }
     RowArgs<T> rowargs(const void *src, long long ss, void *dst, long long ds, long long nrows, double scale,
                        int op, int n)
@@ -229,18 +229,18 @@ template <typename T> struct Ops {
         RowArgs<T> a{};
         a.src = src; a.dst = dst; a.src_stride = ss; a.dst_stride = ds; a.npairs = nrows / 2;
         a.scale = (T)scale; a.ktab = ctx->d_kx;
-        tables(op, n, a.twF, a.twB, ROLE_TP);
+        tables(op, n, a.twF, a.twB);
         a.pad_scale = (T)1; a.pad_mode = 0;
         return a;
     }
     ColArgs<T> colargs(const void *src, long long srow, long long spl, void *dst, long long drow, long long dpl,
-                       int ncols, int nlev, double scale, int op, int n, int family = ROLE_TP)
+                       int ncols, int nlev, double scale, int op, int n)
     {
         ColArgs<T> a{};
         a.src = src; a.dst = dst; a.src_row = srow; a.dst_row = drow; a.src_plane = spl; a.dst_plane = dpl;
         a.ncols = ncols; a.nlev = nlev; a.scale = (T)scale; a.ktab = ctx->d_ky1;
-        tables(op, n, a.twF, a.twB, family);
-        a.pad_copy = 0; a.zero_nyq = 0; a.kmul = 0;
+        tables(op, n, a.twF, a.twB);
+        a.pad_copy = 0; a.zero_nyq = 0;
         return a;
     }
 
@@ -387,13 +387,9 @@ template <typename T> struct Ops {
         return cols(OP_FWD, false, ctx->nyt, ca, "fftn_cols");
     }
     // complex planes -> real planes; tmp receives the y-inverse (may alias in when in is scratch)
-    int ifftn(const C2<T> *in, C2<T> *tmp, T *out, long long out_plane_off_unused, int nlev, int kmul,
-              T pad_scale = (T)1, int pad_mode = 0)
+    int ifftn(const C2<T> *in, C2<T> *tmp, T *out, int nlev, T pad_scale = (T)1, int pad_mode = 0)
     {
-        (void)out_plane_off_unused;
         auto ca = colargs(in, ctx->lhx, ctx->sp(), tmp, ctx->lhx, ctx->sp(), ctx->lhx, nlev, 1.0, OP_INV, ctx->nyt);
-        ca.kmul = kmul;
-        ca.ktab = kmul == 1 ? ctx->d_kx : ctx->d_ky2;
         int rc = cols(OP_INV, false, ctx->nyt, ca, "ifftn_cols");
         if (rc) return rc;
         auto ra = rowargs(tmp, ctx->lhx, out, ctx->ldx, (long long)ctx->nyt * nlev, 1.0, OP_INV, ctx->nxt);
@@ -409,7 +405,7 @@ template <typename T> struct Ops {
         C2<T> *sp = (C2<T> *)ctx->tmp.p;
         const double cst = 1.0 / ((double)ctx->nxt * ctx->nyt);   // 006_test_filter.f90:98
         if ((rc = fftn(f, sp, nlev, cst))) return rc;
-        return ifftn(sp, sp, f, 0, nlev, 0, (T)cst, 1);
+        return ifftn(sp, sp, f, nlev, (T)cst, 1);
     }
 
     // ---- press_stag_array (109_press_stag_array.f90:107-240) ----
@@ -713,41 +709,34 @@ template <typename T> struct Ops {
     }
 
     // ---- divstress_uv / divstress_w (107_divstress.f90:4-104), single-rank roles ----
-    // ddx(tx) into divt's computed levels, then the ddy(ty) column pass whose stores add
-    // it, the vertical difference of tz and the zero pads; BOGUS on the other levels.
+    // ddy(ty) into divt's computed levels, then the ddx(tx) row pass whose stores add it, the
+    // vertical difference of tz and the zero pads; BOGUS on the other levels.
     // bottom / top: the rank holds the wall / the top of the domain (coordz == 0 /
     // coordz == npz-1); a whole domain holds both
     int divstress(T *divt, const T *tx, const T *ty, const T *tz, bool w_form, bool bottom = true, bool top = true)
     {
         const int nz = ctx->nz, nlev = (w_form && top) ? nz : nz - 1;   // levels 1..nlev
         const long long pl = ctx->plane();
-        auto ra = rowargs(tx + pl, ctx->ldx, divt + pl, ctx->ldx, (long long)ctx->nyt * nlev, 1.0 / ctx->nxt,
-                          OP_DERIV, ctx->nxt);
-        ra.ktab = ctx->d_kx;
-        int rc = rows(OP_DERIV, ctx->nxt, ra, "divt_ddx_rows");
-        if (rc) return rc;
         auto ca = colargs(ty + pl, ctx->ldx, pl, divt + pl, ctx->ldx, pl, ctx->nxt, nlev, 1.0 / ctx->nyt, OP_DERIV,
-                          ctx->nyt, 0);
-        ca.ktab = ctx->d_ky1;
-        DivEpi<T> ep{};
+                          ctx->nyt);
+        int rc = cols(OP_DERIV, true, ctx->nyt, ca, "divt_ddy_cols");
+        if (rc) return rc;
+        auto ra = rowargs(tx + pl, ctx->ldx, nullptr, ctx->ldx, (long long)ctx->nyt * nlev, 1.0 / ctx->nxt, OP_DERIV,
+                          ctx->nxt);
+        DivRows<T> ep{};
         ep.out = divt + pl;
         ep.tz = tz + pl;
-        ep.row = ctx->ldx;
         ep.plane = pl;
-        ep.ncols = ctx->nxt;
+        ep.ny = ctx->nyt;
         ep.rdz = (T)(1.0 / ctx->dz);
         ep.fwd = w_form ? 0 : 1;
         ep.zlo = (w_form && bottom) ? 1 : 0;  // divstress_w: no dz(tzz) on the wall level (:81-88)
         ep.zhi = w_form ? nz - 2 : nlev - 1;  // ... nor on the top level (:97-98)
-        {
-            LaunchScope ls(ctx->rec, "divt_ddy_cols", s());
-            if ((rc = chk(launch_cols_divt<T>(ctx->nyt, ca, ep, s()), "divt_ddy_cols"))) return rc;
-        }
-        cudaError_t e = cudaSuccess;
-        LaunchScope ls(ctx->rec, "divt_bogus", s());
-        launch_fill<T>(divt, pl, (T)-1234567890.0, s(), e);   // BOGUS, 001_param.f90:40
-        if (!w_form || !top) launch_fill<T>(divt + pl * nz, pl, (T)-1234567890.0, s(), e);   // :42, :101
-        return chk(e, "divt_bogus");
+        ep.bogus[0] = divt;
+        ep.bogus[1] = !w_form || !top ? divt + pl * nz : nullptr;   // :42, :101
+        ep.bogus_value = (T)-1234567890.0;                         // BOGUS, 001_param.f90:40
+        LaunchScope ls(ctx->rec, "divt_ddx_rows", s());
+        return chk(launch_rows_divt<T>(ctx->nxt, ra, ep, s()), "divt_ddx_rows");
     }
 
     // ---- the fused step ----
@@ -2040,7 +2029,7 @@ int obl_ifftn_dev(obl_ctx *ctx, const void *in, void *out, int nlev)
     DEVCALL(ctx, {
         int rc = ensure(ctx, ctx->tmp, sizeof(C2<T>) * (size_t)ctx->sp() * nlev);
         if (rc) return rc;
-        return o.ifftn((const C2<T> *)in, (C2<T> *)ctx->tmp.p, (T *)out, 0, nlev, 0);
+        return o.ifftn((const C2<T> *)in, (C2<T> *)ctx->tmp.p, (T *)out, nlev);
     });
 }
 int obl_zero_padding_dev(obl_ctx *ctx, const void *var, void *big, int nlev)
@@ -2168,7 +2157,7 @@ int obl_ifftn(obl_ctx *ctx, const double *in, double *out, int nlev)
     HOSTCALL(double, ctx, a, {
         int rc = ensure(ctx, ctx->tmp, sizeof(C2<T>) * (size_t)ctx->sp() * nlev);
         if (rc) return rc;
-        return o.ifftn((const C2<T> *)d[0], (C2<T> *)ctx->tmp.p, (T *)d[1], 0, nlev, 0);
+        return o.ifftn((const C2<T> *)d[0], (C2<T> *)ctx->tmp.p, (T *)d[1], nlev);
     });
 }
 int obl_zero_padding(obl_ctx *ctx, const double *var, double *big, int nlev)

@@ -36,34 +36,74 @@ template <typename T, bool FIRST> struct GSrc {
     }
 };
 
-template <typename T, int N, int NW, int WB, bool TWG, bool FIRST>
-__global__ void __launch_bounds__(32 * NW, col_min_blocks(TWG)) k_cols_gform(ColArgs<T> a, GSrc<T, FIRST> g)
+// A CTA owns WB adjacent complex columns of one plane.  Lane l % WB is the line, the other
+// lane bits and the warp index are the butterfly slot (LL slots), and the exchange is
+// line-minor; a three-radix plan (fft2.cuh).  The two-pass columns measured slower here: G
+// takes three loads an element, which a radix-32 butterfly's registers do not leave in
+// flight (512 lines FP64, 64 levels: 138 us against 224).  FP32 lines of 256 and more read
+// their twiddles through L1, with the registers bounded for 4 CTAs an SM.
+constexpr int kGformWarps = 8;
+template <typename T> struct GformGeo {
+    static constexpr int WB = sizeof(T) == 4 ? 8 : 4, LL = (32 / WB) * kGformWarps;
+};
+template <typename T, int N> constexpr bool gform_tw_global() { return sizeof(T) == 4 && N >= 256; }
+
+template <typename T, int N, bool FIRST>
+__global__ void __launch_bounds__(32 * kGformWarps, gform_tw_global<T, N>() ? 4 : 1) k_cols_gform(ColArgs<T> a, GSrc<T, FIRST> g)
 {
     using C = C2<T>;
     using D = LineDerived<N, OP_FWD>;
+    constexpr int WB = GformGeo<T>::WB, LL = GformGeo<T>::LL, VR = Regs<N, LL, typename D::PF>::v;
+    using G0 = Geo<N, D::RF0, LL>;
+    using GL = Geo<N, D::RFL, LL>;
     extern __shared__ __align__(16) unsigned char smraw[];
-    if constexpr (TWG) {
-        cols2_unit<T, N, OP_FWD, false, NW, WB, NoColEpi, GSrc<T, FIRST>>(
-            a, blockIdx.x, blockIdx.y, a.twF, a.twB, reinterpret_cast<C *>(smraw), NoColEpi(), g);
-    } else {
-        C *twF = reinterpret_cast<C *>(smraw);
-        C *buf = twF + D::TF + D::TB;
-        load_tables<T, N, OP_FWD>(a.twF, a.twB, twF, twF + D::TF);
+    C *buf = reinterpret_cast<C *>(smraw);
+    const C *tw = a.twF;
+    if constexpr (!gform_tw_global<T, N>()) {
+        C *s = buf;
+        buf += D::TF;
+        for (int i = threadIdx.x; i < D::TF; i += blockDim.x) s[i] = a.twF[i];
         __syncthreads();
-        cols2_unit<T, N, OP_FWD, false, NW, WB, NoColEpi, GSrc<T, FIRST>>(a, blockIdx.x, blockIdx.y, twF,
-                                                                                 twF + D::TF, buf, NoColEpi(), g);
+        tw = s;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, z = blockIdx.y;
+    const int line = lane % WB, t = lane / WB + (32 / WB) * warp, gl = blockIdx.x * WB + line;
+    const bool act = gl < a.ncols;
+    LineMinor<C, WB> sc{buf, line};
+    C v[VR];
+#pragma unroll
+    for (int b = 0; b < G0::PER; ++b) {
+        const int j = t + LL * b;
+#pragma unroll
+        for (int r = 0; r < D::RF0; ++r)
+            v[b * D::RF0 + r] = act && (G0::FULL || j < G0::NB) ? g(z, j + r * G0::NB, gl) : mk<T>(0, 0);
+    }
+    fft_regs<N, typename D::PF, LL, true, true>(v, sc, tw, t);
+    if (!act) return;
+    C *dst = reinterpret_cast<C *>(a.dst) + (long long)z * a.dst_plane;
+#pragma unroll
+    for (int b = 0; b < GL::PER; ++b) {
+        const int j = t + LL * b;
+        if (GL::FULL || j < GL::NB)
+#pragma unroll
+            for (int r = 0; r < D::RFL; ++r) {
+                const int i = j + r * GL::NB;
+                // the checked build tests each element's level, column and plane offset
+                if (!(ck_in(z, a.nlev, CK_COL_STORE) && ck_in(gl, a.dst_row, CK_COL_STORE) &&
+                      ck_in((long long)i * a.dst_row + gl, a.dst_plane, CK_COL_STORE)))
+                    continue;
+                dst[(long long)i * a.dst_row + gl] = a.zero_nyq && i == N / 2 ? mk<T>(0, 0) : v[b * D::RFL + r];
+            }
     }
 }
 
-// the same CTA shape and shared memory as the plain y-transform of the RHS spectra
 template <typename T, int N, bool FIRST>
 static cudaError_t gform_launch(const ColArgs<T> &a, const GSrc<T, FIRST> &g, cudaStream_t s)
 {
-    constexpr int NW = 8, WB = LmGeo<T>::WB;
-    constexpr bool TWG = col_tw_global<T, N>();
     using D = LineDerived<N, OP_FWD>;
-    const size_t sm = TWG ? sizeof(C2<T>) * (size_t)D::NM * WB : cols2_smem<T, N, OP_FWD, WB>();
-    auto kern = k_cols_gform<T, N, NW, WB, TWG, FIRST>;
+    constexpr int WB = GformGeo<T>::WB;
+    const size_t sm = sizeof(C2<T>) * ((gform_tw_global<T, N>() ? 0 : (size_t)D::TF) + (size_t)N * WB);
+    auto kern = k_cols_gform<T, N, FIRST>;
     static bool inits[kMaxDevices] = {};
     const int ds = device_slot();
     if (ds < 0 || !inits[ds]) {
@@ -73,7 +113,7 @@ static cudaError_t gform_launch(const ColArgs<T> &a, const GSrc<T, FIRST> &g, cu
     }
     dim3 grid((a.ncols + WB - 1) / WB, a.nlev);
     if (grid.x < 1 || grid.y < 1) return cudaSuccess;
-    kern<<<grid, 32 * NW, sm, s>>>(a, g);
+    kern<<<grid, 32 * kGformWarps, sm, s>>>(a, g);
     return cudaGetLastError();
 }
 

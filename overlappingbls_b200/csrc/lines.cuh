@@ -55,11 +55,10 @@ template <typename T> struct ColArgs {
     int ncols;                       // real columns (real ops) / complex columns
     int nlev;
     T scale;                         // multiplies the input at load
-    const double *ktab;              // DERIV: k[0..N/2]; INV kmul=1: kx per column; kmul=2: ky per row
+    const double *ktab;              // DERIV: k[0..N/2]
     const C2<T> *twF, *twB;
     int pad_copy;                    // UNPAD: also write columns 0,1 into ncols, ncols+1
     int zero_nyq;                    // FWD: zero the Nyquist row (203_fftn_mpi.f90:33)
-    int kmul;                        // INV: 0 none, 1 multiply by i*kx(col), 2 by i*ky(row)
     int pf_ahead;                    // the unit of plane z also prefetches its input lines of
                                      // plane z + pf_ahead into L2 (0 = none)
     int tma;                         // FP32 y-pad: input tile by tensor-map copies (k_tp_cols_tma)
@@ -236,8 +235,9 @@ __device__ __forceinline__ void col_unit(const ColArgs<T> &a, int z, int tx, con
     C v[VR];
     T cr = 0, ci = 0;
 
+    static_assert(OP != OP_INV, "forward passes only");
     auto body = [&](auto &acc) {
-        if constexpr (OP != OP_INV) {
+        {
             using G = Geo<NI, D::RF0, LL>;
             if constexpr (REAL) {
                 const C c0v = acc.ld(0);
@@ -278,29 +278,6 @@ __device__ __forceinline__ void col_unit(const ColArgs<T> &a, int z, int tx, con
         } else {
             C w[VR];
             C *vb = v;
-            if constexpr (OP == OP_INV) {
-                using G = Geo<NO, D::RB0, LL>;
-#pragma unroll
-                for (int b = 0; b < G::PER; ++b) {
-                    const int j = t + LL * b;
-#pragma unroll
-                    for (int r = 0; r < D::RB0; ++r) {
-                        const int i = j + r * G::NB;
-                        C x = mk<T>(0, 0);
-                        if (G::FULL || j < G::NB) {
-                            x = acc.ld(i);
-                            if (a.kmul) {
-                                const T kk = (T)(a.kmul == 1 ? a.ktab[c0 + cc] : a.ktab[i]);
-                                x = mk<T>(-kk * x.y, kk * x.x);
-                            }
-                            x.x *= a.scale;
-                            x.y *= a.scale;
-                        }
-                        v[b * D::RB0 + r] = x;
-                    }
-                }
-                __syncwarp();
-            }
             if constexpr (OP == OP_DERIV) reg_deriv<T, N, D::RFL, LL>(v, a.ktab, t);
             if constexpr (OP == OP_PAD) { reg_pad<T, N, D::RFL, LL>(v, w, t); vb = w; }
             if constexpr (OP == OP_UNPAD) { reg_unpad<T, N, D::RB0, LL>(v, w, t); vb = w; }
@@ -347,205 +324,9 @@ __device__ __forceinline__ void col_unit(const ColArgs<T> &a, int z, int tx, con
     __syncthreads();   // the tile may be reused by the caller's next unit
 }
 
-// ----------------------------------------------------------------------------- line-minor columns
-// Column lines without a staging tile: a CTA owns WB adjacent complex lines (WB real
-// column pairs, or WB complex columns) of one plane.  Lane l % WB is the line and the
-// remaining lane bits and the warp index form the butterfly slot t (LL slots), so
-//   * the first pass loads its operands straight from global memory: for every element
-//     index the WB lanes of a line group read WB adjacent pairs (coalesced, 8/16-byte
-//     vector loads), and the last pass stores the same way;
-//   * the exchange scratch is line-minor (element i of line l at buf[i*WB + l]): a warp
-//     always touches consecutive words, so no pass has bank conflicts;
-//   * passes are separated by __syncthreads() because a line spans all warps.
-template <typename T, int NW_ = 8, int WB_ = (sizeof(T) == 4 ? 8 : 4)> struct LmGeo {
-    static constexpr int WB = WB_;                        // lines per CTA (WB*8-byte row segments)
-    static constexpr int NW = NW_;                        // warps per CTA
-    static constexpr int LL = (32 / WB) * NW;             // butterfly slots per line
-};
-// Shape of the three-radix column kernels that remain beside the two-pass ones below (the G
-// form and the stress divergence, whose load and store hooks hold more registers than a
-// radix-32 butterfly leaves): 8 warps a CTA; FP32 lines of 256 and more read their twiddles
-// through L1, with the registers bounded for 32 warps an SM.
 #ifndef OBL_COL_PF
 #define OBL_COL_PF 2   // y-pad column kernel: L2 prefetch distance in quarters of a residency window (0 = off)
 #endif
-template <typename T, int N> constexpr bool col_tw_global() { return sizeof(T) == 4 && N >= 256; }
-constexpr int col_min_blocks(bool twg) { return twg ? 4 : 1; }
-
-template <typename T, int N, int OP, int NW = 8, int WB = LmGeo<T>::WB> struct ColDerived {
-    using D = LineDerived<N, OP>;
-    static constexpr int LL = LmGeo<T, NW, WB>::LL;
-    static constexpr int rf = Regs<D::NI, LL, typename D::PF>::v, rb = Regs<D::NO, LL, typename D::PB>::v;
-    static constexpr int VR = rf > rb ? rf : rb;
-};
-
-// Store hook of the column kernel's backward output: epi(z, i, line, x) may change the
-// value x of row i, line `line` of plane z just before it is stored; epi.prefetch(z, i,
-// line) is called for the same elements when the line is loaded, before its transforms,
-// so that what the hook reads is on chip by the time it is stored.  The default does
-// nothing and compiles away.
-struct NoColEpi {
-    template <class C> __device__ __forceinline__ void operator()(int, int, int, C &) const {}
-    __device__ __forceinline__ void prefetch(int, int, int) const {}
-};
-
-// Load hook of the column kernel's input: src(z, i, line) returns element i of global line
-// `line` of plane z in place of the plain load from a.src.  The default is the plain load.
-struct NoColSrc {};
-
-// One CTA unit of the line-minor column kernel: line group bx of plane z.  The plan
-// tables twF/twB are already in shared memory; buf is the exchange scratch (NM*WB).
-// Called by the column kernels with hooks (gform.cu, divstress.cu) and by the persistent
-// ensemble kernel.
-template <typename T, int N, int OP, bool REAL, int NW = 8, int WB_ = LmGeo<T>::WB, class EPI = NoColEpi,
-          class SRC = NoColSrc>
-__device__ __forceinline__ void cols2_unit(const ColArgs<T> &a, int bx, int z, const C2<T> *twF,
-                                           const C2<T> *twB, C2<T> *buf, const EPI &epi = EPI(),
-                                           const SRC &src = SRC())
-{
-    using C = C2<T>;
-    using E = typename std::conditional<REAL, T, C>::type;
-    using D = LineDerived<N, OP>;
-    using G = LmGeo<T, NW, WB_>;
-    constexpr int NI = D::NI, NO = D::NO, WB = G::WB, LL = G::LL, VR = ColDerived<T, N, OP, NW, WB_>::VR;
-    (void)NI;
-    (void)twF;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int line = lane % WB, t = lane / WB + (32 / WB) * warp;
-    const int gl = bx * WB + line;                         // global line index
-    const int nlines = REAL ? a.ncols / 2 : a.ncols;
-    const bool act = gl < nlines;
-    const int glc = act ? gl : 0;
-    // element i of this line: a complex value (a real column pair for REAL)
-    const E *srcz = reinterpret_cast<const E *>(a.src) + (long long)z * a.src_plane;
-    E *dstz = reinterpret_cast<E *>(a.dst) + (long long)z * a.dst_plane;
-    // the checked build tests each element's level, column and plane offset against the
-    // extents the arguments give (nlev planes of src_plane / dst_plane, rows of src_row / dst_row)
-    auto col_ok = [&](int i, int col, int row, long long plane, int site) {
-        const int ce = REAL ? 2 * col + 1 : col;
-        return ck_in(z, a.nlev, site) && ck_in(ce, row, site) && ck_in((long long)i * row + ce, plane, site);
-    };
-    auto gld = [&](int i) -> C {
-        if constexpr (!std::is_same<SRC, NoColSrc>::value) return src(z, i, glc);
-        else {
-            if (OBL_CHECK && !col_ok(i, glc, a.src_row, a.src_plane, CK_COL_LOAD)) return mk<T>(0, 0);
-            if constexpr (REAL) return __ldcg(reinterpret_cast<const C *>(srcz + (long long)i * a.src_row + 2 * glc));
-            else return __ldcg(srcz + (long long)i * a.src_row + glc);
-        }
-    };
-    auto gst = [&](int i, C v) {
-        if (OBL_CHECK && !col_ok(i, gl, a.dst_row, a.dst_plane, CK_COL_STORE)) return;
-        if constexpr (REAL) *reinterpret_cast<C *>(dstz + (long long)i * a.dst_row + 2 * gl) = v;
-        else dstz[(long long)i * a.dst_row + gl] = v;
-    };
-    LineMinor<C, WB> sc{buf, line};
-    C v[VR];
-    C cref = mk<T>(0, 0);
-
-    if constexpr (OP != OP_INV) {
-        using GG = Geo<NI, D::RF0, LL>;
-        if constexpr (REAL) cref = gld(0);
-#pragma unroll
-        for (int b = 0; b < GG::PER; ++b) {
-            const int j = t + LL * b;
-#pragma unroll
-            for (int r = 0; r < D::RF0; ++r) {
-                C x = mk<T>(0, 0);
-                if (act && (GG::FULL || j < GG::NB)) {
-                    x = gld(j + r * GG::NB);
-                    x.x = (x.x - cref.x) * a.scale;
-                    x.y = (x.y - cref.y) * a.scale;
-                }
-                v[b * D::RF0 + r] = x;
-            }
-        }
-        if constexpr (!std::is_same<EPI, NoColEpi>::value) {
-            using GP = Geo<NO, D::RBL, LL>;
-            if (act) {
-#pragma unroll
-                for (int b = 0; b < GP::PER; ++b) {
-                    const int j = t + LL * b;
-                    if (GP::FULL || j < GP::NB)
-#pragma unroll
-                        for (int r = 0; r < D::RBL; ++r) epi.prefetch(z, j + r * GP::NB, gl);
-                }
-            }
-        }
-        fft_regs<NI, typename D::PF, LL, true, true>(v, sc, twF, t);
-    }
-    if constexpr (OP == OP_FWD) {
-        using GG = Geo<NI, D::RFL, LL>;
-        if (act) {
-#pragma unroll
-            for (int b = 0; b < GG::PER; ++b) {
-                const int j = t + LL * b;
-                if (GG::FULL || j < GG::NB)
-#pragma unroll
-                    for (int r = 0; r < D::RFL; ++r) {
-                        const int i = j + r * GG::NB;
-                        C x = v[b * D::RFL + r];
-                        if (a.zero_nyq && i == NI / 2) x = mk<T>(0, 0);
-                        gst(i, x);
-                    }
-            }
-        }
-    } else {
-        C w[VR];
-        C *vb = v;
-        if constexpr (OP == OP_INV) {
-            using GG = Geo<NO, D::RB0, LL>;
-#pragma unroll
-            for (int b = 0; b < GG::PER; ++b) {
-                const int j = t + LL * b;
-#pragma unroll
-                for (int r = 0; r < D::RB0; ++r) {
-                    const int i = j + r * GG::NB;
-                    C x = mk<T>(0, 0);
-                    if (act && (GG::FULL || j < GG::NB)) {
-                        x = gld(i);
-                        if (a.kmul) {
-                            const T kk = (T)(a.kmul == 1 ? a.ktab[glc] : a.ktab[i]);
-                            x = mk<T>(-kk * x.y, kk * x.x);
-                        }
-                        x.x *= a.scale;
-                        x.y *= a.scale;
-                    }
-                    v[b * D::RB0 + r] = x;
-                }
-            }
-        }
-        if constexpr (OP == OP_DERIV) reg_deriv<T, N, D::RFL, LL>(v, a.ktab, t);
-        if constexpr (OP == OP_PAD) { reg_pad<T, N, D::RFL, LL>(v, w, t); vb = w; }
-        if constexpr (OP == OP_UNPAD) { reg_unpad<T, N, D::RB0, LL>(v, w, t); vb = w; }
-        fft_regs<NO, typename D::PB, LL, false, true>(vb, sc, twB, t);
-        using GG = Geo<NO, D::RBL, LL>;
-        const bool addc = (OP == OP_PAD || OP == OP_UNPAD);
-        if (act) {
-#pragma unroll
-            for (int b = 0; b < GG::PER; ++b) {
-                const int j = t + LL * b;
-                if (GG::FULL || j < GG::NB)
-#pragma unroll
-                    for (int r = 0; r < D::RBL; ++r) {
-                        const int i = j + r * GG::NB;
-                        C x = vb[b * D::RBL + r];
-                        if (addc) {
-                            x.x += cref.x;
-                            x.y += cref.y;
-                        }
-                        epi(z, i, gl, x);
-                        gst(i, x);
-                        if constexpr (OP == OP_UNPAD && REAL) {
-                            // var(nxt+1:ldx,:) = var(1:2,:) (108_01_padd.f90:195)
-                            if (a.pad_copy && gl == 0 && ck_in(a.ncols + 1, a.dst_row, CK_COL_STORE))
-                                *reinterpret_cast<C *>(dstz + (long long)i * a.dst_row + a.ncols) = x;
-                        }
-                    }
-            }
-        }
-    }
-}
-
 // ----------------------------------------------------------------------------- two-pass columns
 // Geometry of a line operation: RI, RO the second radices of its input and output
 // transforms, PI and PO the pitches of their exchanges, ROWS the exchange rows of one line
@@ -576,17 +357,15 @@ __device__ __forceinline__ void tp_deriv(C2<T> (&v)[R1], const double *ktab, int
 // lanes of a butterfly read and store WB adjacent pairs; the exchange is line-minor
 // (element row e of line l at buf[e*WB + l]).
 // SMEM_IN: the unit's input is already in buf, row i of line l at buf[i*WB + l].
-template <typename T, int N, int OP, bool REAL, int NT, int WB, class EPI = NoColEpi, bool SMEM_IN = false,
-          class SRC = NoColSrc>
-__device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z, C2<T> *buf, const EPI &epi = EPI(),
-                                             const SRC &src = SRC())
+template <typename T, int N, int OP, bool REAL, int NT, int WB, bool SMEM_IN = false>
+__device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z, C2<T> *buf)
 {
     using C = C2<T>;
     using E = typename std::conditional<REAL, T, C>::type;
     using D = TpLine<N, OP>;
     constexpr int R0 = D::R0, RI = D::RI, RO = D::RO;
     constexpr int I1 = RI * WB, I2 = R0 * WB, I3 = RO * WB;       // butterflies of the three mappings
-    constexpr int PER1 = (I1 + NT - 1) / NT, PER2 = I2 / NT, PER3 = (I3 + NT - 1) / NT;
+    constexpr int PER1 = (I1 + NT - 1) / NT, PER2 = I2 / NT;
     static_assert(NT % WB == 0 && I2 % NT == 0, "whole butterflies per thread in the middle passes");
     static_assert(!SMEM_IN || PER1 == 1, "an input tile is read before its exchange overwrites it");
     const int tid = threadIdx.x, line = tid % WB;
@@ -603,8 +382,7 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
         return ck_in(z, a.nlev, site) && ck_in(ce, row, site) && ck_in((long long)i * row + ce, plane, site);
     };
     auto gld = [&](int i) -> C {
-        if constexpr (!std::is_same<SRC, NoColSrc>::value) return src(z, i, glc);
-        else if constexpr (SMEM_IN) return buf[i * WB + line];
+        if constexpr (SMEM_IN) return buf[i * WB + line];
         else {
             if (OBL_CHECK && !col_ok(i, glc, a.src_row, a.src_plane, CK_COL_LOAD)) return mk<T>(0, 0);
             if constexpr (REAL) return __ldcg(reinterpret_cast<const C *>(srcz + (long long)i * a.src_row + 2 * glc));
@@ -675,17 +453,6 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
                 for (int r = 0; r < R0; ++r) buf[(j * D::PI + r) * WB + line] = x[r];
             }
         }
-        if constexpr (!std::is_same<EPI, NoColEpi>::value) {
-            if (act) {
-#pragma unroll
-                for (int b = 0; b < PER3; ++b) {
-                    const int f = tid + b * NT, j = f / WB;
-                    if (I3 % NT == 0 || f < I3)
-#pragma unroll
-                        for (int r = 0; r < R0; ++r) epi.prefetch(z, j + r * RO, gl);
-                }
-            }
-        }
         __syncthreads();
 #pragma unroll
         for (int b = 0; b < PER2; ++b) {
@@ -713,10 +480,6 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
             for (int r = 0; r < RO; ++r) {
                 const int i = j + r * R0;
                 C x = act ? gld(i) : mk<T>(0, 0);
-                if (a.kmul) {
-                    const T kk = (T)(a.kmul == 1 ? a.ktab[glc] : a.ktab[i]);
-                    x = mk<T>(-kk * x.y, kk * x.x);
-                }
                 v[b][r] = cscale(x, a.scale);
             }
         }
@@ -769,7 +532,6 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
                         y.x += cref.x;
                         y.y += cref.y;
                     }
-                    epi(z, i, gl, y);
                     gst(i, y);
                     if constexpr (OP == OP_UNPAD && REAL) {
                         // var(nxt+1:ldx,:) = var(1:2,:) (108_01_padd.f90:195)
@@ -1161,7 +923,7 @@ __global__ void __launch_bounds__(TpGeo<T, N, OP>::NT, TpGeo<T, N, OP>::minb)
         if (a.wait_err) atomicExch(a.wait_err, 1);
         mbar_wait_bounded(sbar, 0);   // a late copy lands before the tile is reused
     }
-    tp_cols_unit<T, N, OP, REAL, TpGeo<T, N, OP>::NT, WB, NoColEpi, true>(a, blockIdx.x, blockIdx.y, buf);
+    tp_cols_unit<T, N, OP, REAL, TpGeo<T, N, OP>::NT, WB, true>(a, blockIdx.x, blockIdx.y, buf);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link)
@@ -1212,12 +974,6 @@ template <typename T, int N, int OP> cudaError_t launch_rows_t(const RowArgs<T> 
     if (grid < 1) return cudaSuccess;
     kern<<<(unsigned)grid, OP == OP_INV ? G::NTI : G::NT, sm, s>>>(a);
     return cudaGetLastError();
-}
-
-template <typename T, int N, int OP, int WB = LmGeo<T>::WB> inline size_t cols2_smem()
-{
-    using D = LineDerived<N, OP>;
-    return sizeof(C2<T>) * ((size_t)D::TF + D::TB + (size_t)D::NM * WB);
 }
 
 template <typename T, int N, int OP, bool REAL> cudaError_t launch_cols_t(const ColArgs<T> &a0, cudaStream_t s)

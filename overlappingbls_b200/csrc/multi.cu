@@ -1,6 +1,6 @@
 // multi.cu -- the row and column line kernels over several fields of one shape in one
 // launch (see launch_rows_multi / launch_cols_multi in lines.cuh).  The per-line work is
-// row_unit / cols2_unit unchanged; only the field of each unit is looked up first.
+// tp_row_unit / tp_cols_unit unchanged; only the field of each unit is looked up first.
 #include "lines_dispatch.cuh"
 
 namespace obl {
