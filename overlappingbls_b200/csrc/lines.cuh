@@ -29,7 +29,8 @@
 
 namespace obl {
 
-enum LineOp : int { OP_DERIV = 0, OP_PAD = 1, OP_UNPAD = 2, OP_FWD = 3, OP_INV = 4 };
+// (OP_FILT: forward and backward on complex columns, the Nyquist bin dropped between)
+enum LineOp : int { OP_DERIV = 0, OP_PAD = 1, OP_UNPAD = 2, OP_FWD = 3, OP_INV = 4, OP_FILT = 5 };
 // twiddle tables of a length: the three-radix plans of fft2.cuh, and (+ ROLE_TP) the
 // two-pass ones of twopass.cuh
 enum PlanRole : int { ROLE_FWD = 0, ROLE_BWD = 1, ROLE_PADFWD = 2, ROLE_PADBWD = 3, ROLE_TP = 4 };
@@ -507,6 +508,7 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
                 DftPad<D::R1>::run(v[b], [&](auto ic, C x) { buf[(j * D::PO + decltype(ic)::value) * WB + line] = x; });
             } else {
                 if constexpr (OP == OP_DERIV) tp_deriv<T, N, R0, RO>(v[b], a.ktab, j);
+                if constexpr (OP == OP_FILT) if (j == 0) v[b][RO / 2] = mk<T>(0, 0);
                 Dft<RO, false>::run(v[b]);
 #pragma unroll
                 for (int r = 0; r < RO; ++r) buf[(j * D::PO + r) * WB + line] = v[b][r];
@@ -553,8 +555,9 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
 // keep more of them loading (ddy 1.214 against 1.450 ms), which the y-pad's larger exchange
 // does not repay (2.63 against 2.34 ms).
 // Against the three-radix kernels (ms per step at 512x512x256 levels, before -> now): FP32
-// y-pad 1.243 -> 0.846, ddy 0.714 -> 0.571, y-transform 0.393 -> 0.351; FP64 3.00 -> 2.34,
-// 1.85 -> 1.21; at 128x128 levels the y-pad takes 0.62 and the y-unpad 0.55 of their time.
+// y-pad 1.243 -> 0.888, ddy 0.714 -> 0.566, y-transform 0.393 -> 0.358; FP64 y-pad 3.00 ->
+// 2.31, ddy 1.85 -> 1.30; at 128x128 levels the y-pad takes 0.62 and the y-unpad 0.55 of
+// their time.
 // The L1/shared pipe fell from 70 to 55% busy at half the time per byte.  A persistent form
 // with the next tile's copies in flight measured slower (1.25 ms): its second tile leaves
 // shared memory for 16 warps only.

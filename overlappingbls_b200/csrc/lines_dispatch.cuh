@@ -38,6 +38,7 @@ cudaError_t cols_n(int op, bool real, const ColArgs<T> &a, cudaStream_t s)
         switch (op) {
         case OP_FWD: return launch_cols_t<T, N, OP_FWD, false>(a, s);
         case OP_INV: return launch_cols_t<T, N, OP_INV, false>(a, s);
+        case OP_FILT: return launch_cols_t<T, N, OP_FILT, false>(a, s);
         }
     }
     return cudaErrorInvalidValue;
