@@ -20,6 +20,7 @@
 
 #include "common.cuh"
 #include "lines.cuh"
+#include "lines3.cuh"
 #include "press.cuh"
 #include "fused.cuh"
 #include "convec.cuh"
@@ -396,6 +397,36 @@ template <typename T> struct Ops {
         return rows(OP_INV, ctx->nxt, ra, "ifftn_rows");
     }
 
+    // the three-radix FP32 transforms of press_stag_array on real(8) arrays (lines3.cuh)
+    int rows3(int op, int n, RowArgs<T> a, const char *name)
+    {
+        if constexpr (std::is_same<T, float>::value) {
+            a.twF = twt<T>(ctx, n, ROLE_FWD);
+            a.twB = twt<T>(ctx, n, ROLE_BWD);
+            LaunchScope ls(ctx->rec, name, s());
+            return chk(launch_rows3(op, n, a, s()), name);
+        }
+        return OBL_ERR_UNSUPPORTED;
+    }
+    int cols3(int op, int n, ColArgs<T> a, int kmul, const char *name)
+    {
+        if constexpr (std::is_same<T, float>::value) {
+            a.twF = twt<T>(ctx, n, ROLE_FWD);
+            a.twB = twt<T>(ctx, n, ROLE_BWD);
+            LaunchScope ls(ctx->rec, name, s());
+            return chk(launch_cols3(op, n, a, kmul, s()), name);
+        }
+        return OBL_ERR_UNSUPPORTED;
+    }
+    int ifftn3(const C2<T> *in, C2<T> *tmp, T *out, int nlev, int kmul)
+    {
+        auto ca = colargs(in, ctx->lhx, ctx->sp(), tmp, ctx->lhx, ctx->sp(), ctx->lhx, nlev, 1.0, OP_INV, ctx->nyt);
+        ca.ktab = kmul == 1 ? ctx->d_kx : ctx->d_ky2;
+        if (int rc = cols3(OP_INV, ctx->nyt, ca, kmul, "ifftn_cols")) return rc;
+        return rows3(OP_INV, ctx->nxt, rowargs(tmp, ctx->lhx, out, ctx->ldx, (long long)ctx->nyt * nlev, 1.0, OP_INV, ctx->nxt),
+                     "ifftn_rows");
+    }
+
     // fftn and ifftn with the column passes of both in one (filter_cols): the y-spectrum is
     // neither stored nor read, three launches in place of four.  One call, before -> now:
     // FP32 160x128x65 levels 49.4 -> 43.3 us, 256x256x257 233 -> 208 us; FP64 64x64x18
@@ -424,10 +455,18 @@ template <typename T> struct Ops {
     // forward kernel); only the boundary planes H_z(0), H_z(nz) are transformed here.
     // proj: when given (with dpdz_out), the inverse is fused with project() on proj->u,v,w
     // stress_free: overrides the context's ubc_stress_free for that project() (-1: keep)
+    // real8: the results go to real(8) host arrays; with FP32 storage the transforms are the
+    // three-radix ones and the islands whole columns (lines3.cuh)
     int press(const T *u, const T *v, const T *w, const T *dbot, const T *dtop, T *p, T *dpdx, T *dpdy,
               T *dpdz_out = nullptr, bool rhs_ready = false, const obl_step_io *proj = nullptr,
-              int stress_free = -1)
+              int stress_free = -1, bool real8 = false)
     {
+        const bool three = real8 && std::is_same<T, float>::value;
+        auto frows = [&](RowArgs<T> ra) -> int { return three ? rows3(OP_FWD, ctx->nxt, ra, "press_fwd_rows") : rows(OP_FWD, ctx->nxt, ra, "press_fwd_rows"); };
+        auto fcols = [&](ColArgs<T> ca, const char *name) -> int {
+            ca.zero_nyq = 1;
+            return three ? cols3(OP_FWD, ctx->nyt, ca, 0, name) : cols(OP_FWD, false, ctx->nyt, ca, name);
+        };
         const long long S = ctx->sp();
         const size_t sb = sizeof(C2<T>) * (size_t)S * (ctx->nz + 1);
         int rc;
@@ -447,7 +486,15 @@ template <typename T> struct Ops {
             m.src[0] = u + pl; m.src[1] = v + pl; m.src[2] = w + pl;
             m.dst[0] = Hx + S; m.dst[1] = Hy + S; m.dst[2] = Hz + S;
             auto ra = rowargs(nullptr, ldx, nullptr, lhx, (long long)ny * L, sc, OP_FWD, nx);
-            if ((rc = rows_multi(OP_FWD, nx, ra, m, 3, "press_fwd_rows"))) return rc;
+            if (three) {
+                for (int f = 0; f < 3; ++f) {
+                    ra.src = m.src[f];
+                    ra.dst = m.dst[f];
+                    if ((rc = frows(ra))) return rc;
+                }
+            } else if ((rc = rows_multi(OP_FWD, nx, ra, m, 3, "press_fwd_rows"))) {
+                return rc;
+            }
         }
         // boundary planes H_z(0) and H_z(nz) (:186-200); an absent one is zero, and so is its
         // y-transform
@@ -459,7 +506,7 @@ template <typename T> struct Ops {
                 const T *pln = zb ? (top ? dtop : nullptr) : dbot;
                 if (pln) {
                     auto ra = rowargs(pln, ldx, Hz + S * zb, lhx, ny, cst, OP_FWD, nx);
-                    if ((rc = rows(OP_FWD, nx, ra, "press_fwd_rows"))) return rc;
+                    if ((rc = frows(ra))) return rc;
                 } else {
                     CK(cudaMemsetAsync(Hz + S * zb, 0, sizeof(C2<T>) * S, s()));
                 }
@@ -471,11 +518,9 @@ template <typename T> struct Ops {
             // H_y as it is; G = i*kx*H_x + (H_z(z+1) - H_z(z) [+ H_z(0)])/dz formed from the
             // x-spectra and transformed over H_x; H_z at level 0, and at levels 1..L only in
             // the line group of kx = 0 (the (0,0) mode's RHS, the same transform as before)
-            if (!rhs_ready) {
-                auto ca = colargs(Hy + S, lhx, S, Hy + S, lhx, S, lhx, L, 1.0, OP_FWD, ny);
-                ca.zero_nyq = 1;
-                if ((rc = cols(OP_FWD, false, ny, ca, "press_fwd_cols"))) return rc;
-            }
+            if (!rhs_ready &&
+                (rc = fcols(colargs(Hy + S, lhx, S, Hy + S, lhx, S, lhx, L, 1.0, OP_FWD, ny), "press_fwd_cols")))
+                return rc;
             {
                 LaunchScope ls(ctx->rec, "press_gform_cols", s());
                 if ((rc = chk(launch_gform_cols<T>(ny, Hx, Hz, ctx->d_kx, S, lhx, L, ctx->dz, twt<T>(ctx, ny, ROLE_FWD),
@@ -483,14 +528,9 @@ template <typename T> struct Ops {
                               "press_gform_cols")))
                     return rc;
             }
-            if (dbot) {
-                auto ca = colargs(Hz, lhx, S, Hz, lhx, S, lhx, 1, 1.0, OP_FWD, ny);
-                ca.zero_nyq = 1;
-                if ((rc = cols(OP_FWD, false, ny, ca, "press_bnd_cols"))) return rc;
-            }
-            auto c0 = colargs(Hz + S, lhx, S, Hz + S, lhx, S, 1, L, 1.0, OP_FWD, ny);   // column kx = 0
-            c0.zero_nyq = 1;
-            if ((rc = cols(OP_FWD, false, ny, c0, "press_mean_cols"))) return rc;
+            if (dbot && (rc = fcols(colargs(Hz, lhx, S, Hz, lhx, S, lhx, 1, 1.0, OP_FWD, ny), "press_bnd_cols"))) return rc;
+            // column kx = 0
+            if ((rc = fcols(colargs(Hz + S, lhx, S, Hz + S, lhx, S, 1, L, 1.0, OP_FWD, ny), "press_mean_cols"))) return rc;
         } else if (!rhs_ready) {
             // H_x, H_y levels 1..L in one launch, H_z levels 0..L+1 in another
             MultiPtr<T> m{};
@@ -498,16 +538,22 @@ template <typename T> struct Ops {
             m.src[1] = m.dst[1] = Hy + S;
             auto ca = colargs(nullptr, lhx, S, nullptr, lhx, S, lhx, L, 1.0, OP_FWD, ny);
             ca.zero_nyq = 1;
-            if ((rc = cols_multi(OP_FWD, ny, ca, m, 2, "press_fwd_cols"))) return rc;
+            if (three) {
+                for (int f = 0; f < 2; ++f) {
+                    ca.src = ca.dst = m.dst[f];
+                    if ((rc = fcols(ca, "press_fwd_cols"))) return rc;
+                }
+            } else if ((rc = cols_multi(OP_FWD, ny, ca, m, 2, "press_fwd_cols"))) {
+                return rc;
+            }
             ca.src = ca.dst = Hz;
             ca.nlev = L + 2;
-            if ((rc = cols(OP_FWD, false, ny, ca, "press_fwd_cols"))) return rc;
+            if ((rc = fcols(ca, "press_fwd_cols"))) return rc;
         } else {
             for (int zb : {0, L + 1}) {
                 if (!(zb ? top : dbot != nullptr)) continue;
-                auto ca = colargs(Hz + S * zb, lhx, S, Hz + S * zb, lhx, S, lhx, 1, 1.0, OP_FWD, ny);
-                ca.zero_nyq = 1;
-                if ((rc = cols(OP_FWD, false, ny, ca, "press_bnd_cols"))) return rc;
+                if ((rc = fcols(colargs(Hz + S * zb, lhx, S, Hz + S * zb, lhx, S, lhx, 1, 1.0, OP_FWD, ny), "press_bnd_cols")))
+                    return rc;
             }
         }
         // tridiagonal solve per (kx,ky) column
@@ -556,7 +602,7 @@ template <typename T> struct Ops {
                     // the bulk launch
                     IslandArgs isl{nullptr, 0, nullptr, nullptr};
                     bool join_side = false;   // the island launches ran on the side stream
-                    const int ip = isl_parts(ta);
+                    const int ip = three ? 1 : isl_parts(ta);
                     if (ip > 1) {
                         const int seg = (L + ip - 1) / ip, Pn = (L + seg - 1) / seg;
                         const size_t ni = (size_t)ctx->n_isl * L;
@@ -628,6 +674,12 @@ template <typename T> struct Ops {
                 launch_tdma<T>(ta, s(), e);
                 if (e != cudaSuccess) return cuda_fail(ctx, e, "tdma");
             }
+        }
+        if (three) {
+            // p at 0..L, dpdx and dpdy at 1..L, each by its own y-inverse; Hx/Hy/Hz are free
+            if ((rc = ifftn3(ph, Hz, p, L + 1, 0))) return rc;
+            if ((rc = ifftn3(ph + S, Hx, dpdx, L, 1))) return rc;
+            return ifftn3(ph + S, Hy, dpdy, L, 2);
         }
         // inverse transforms (:231-238), p at 0..L, dpdx/dpdy (and the spectral dpdz) at 1..L:
         // one y-inverse pass over p_hat (and the dpdz spectrum), one x-inverse pass over the
@@ -2202,7 +2254,7 @@ int obl_press_stag_array(obl_ctx *ctx, const double *u, const double *v, const d
                         harg_out(dpdy, nd, false, ctx->ldx, ctx->nxt, 0, ny * L)};
     HOSTCALL(double, ctx, a,
              return o.press((const T *)d[0], (const T *)d[1], (const T *)d[2], (const T *)d[3], (const T *)d[4],
-                            (T *)d[5], (T *)d[6], (T *)d[7]););
+                            (T *)d[5], (T *)d[6], (T *)d[7], nullptr, false, nullptr, -1, true););
 }
 int obl_dpdz(obl_ctx *ctx, const double *p, double *dpdz)
 {
