@@ -68,6 +68,9 @@ struct obl_ctx {
     DevBuf cscr;               // c' scratch
     DevBuf isl_c, isl_d;
     DevBuf tmp;                // pad/unpad intermediate, ifftn temporary
+    DevBuf xpad;               // x-padded fields of the batched forward pass, which leaves tmp
+                               // (and graphs captured with it) alone
+    bool xpad_nomem = false;   // their allocation failed: the pass stays field by field
     DevBuf fscr;               // cluster scratch slots of the fused forward kernel
     // rollout problem of the adjoint: small (ldx,nyt,0:nz) and padded work fields, the
     // per-step state checkpoints and the objective's partial sums
@@ -847,7 +850,15 @@ template <typename T> struct Ops {
     int fwd_lines(const obl_step_io *io)
     {
         int rc;
-        if (fwd_batched()) return fwd_batch(io);
+        if (fwd_batched()) {
+            // without the memory for four fields' intermediates one field's still does
+            if ((rc = fwd_spec())) return rc;
+            rc = ensure(ctx, ctx->xpad, 4 * xpad_bytes());
+            if (!rc) return fwd_batch(io);
+            if (rc != OBL_ERR_NOMEM) return rc;
+            ctx->xpad_nomem = true;
+            ctx->err.clear();
+        }
         if ((rc = fwd_prepare())) return rc;
         for (int c = 0; c < 4; ++c)
             if ((rc = fwd_field(io, c))) return rc;
@@ -861,20 +872,18 @@ template <typename T> struct Ops {
     // field's launch fills the GPU and its y-pad has the tensor copies: 512x512x256 (1.6 GB)
     // 4693 / 4630, FP64 10235 / 10001.
     static constexpr size_t kFwdBatchBytes = (size_t)512 << 20;
+    size_t xpad_bytes() const { return sizeof(T) * (size_t)ctx->nxt2 * ctx->nyt * (ctx->nz + 1); }
     bool fwd_batched() const
     {
-        return !ctx->param_fwd_chunk && 4 * sizeof(T) * (size_t)ctx->nxt2 * ctx->nyt * (ctx->nz + 1) <= kFwdBatchBytes;
+        return !ctx->param_fwd_chunk && !ctx->xpad_nomem && 4 * xpad_bytes() <= kFwdBatchBytes;
     }
     int fwd_batch(const obl_step_io *io)
     {
         const int nlev = ctx->nz + 1, nx = ctx->nxt, ny = ctx->nyt, nx2 = ctx->nxt2, ny2 = ctx->nyt2, lhx = ctx->lhx;
         const long long S = ctx->sp(), pl = ctx->plane(), plx = (long long)nx2 * ny, plb = (long long)nx2 * ny2;
-        const size_t sb = sizeof(C2<T>) * (size_t)S * (ctx->nz + 1), xsz = (size_t)plx * nlev;
+        const size_t xsz = (size_t)plx * nlev;
         int rc;
-        for (int i = 0; i < 5; ++i)
-            if ((rc = ensure(ctx, ctx->spec[i], sb))) return rc;
-        if ((rc = ensure(ctx, ctx->tmp, sizeof(T) * xsz * 4))) return rc;
-        T *xb = (T *)ctx->tmp.p;
+        T *xb = (T *)ctx->xpad.p;
         const T *f[4] = {(const T *)io->u, (const T *)io->v, (const T *)io->w, (const T *)io->theta};
         RowsFwd3Args<T> ra{};
         ra.npairs = (long long)ny * nlev / 2; ra.ldx = ctx->ldx; ra.ny = ny; ra.L = ctx->L; ra.z0 = 0;
@@ -906,13 +915,18 @@ template <typename T> struct Ops {
         LaunchScope ls(ctx->rec, "cols_fwd", s());
         return chk(ColsFwdLaunch<T>::run(ny, ca, s()), "cols_fwd");
     }
-    int fwd_prepare()
+    int fwd_spec()
     {
         const size_t sb = sizeof(C2<T>) * (size_t)ctx->sp() * (ctx->nz + 1);
         int rc;
         for (int i = 0; i < 5; ++i)
             if ((rc = ensure(ctx, ctx->spec[i], sb))) return rc;
-        return ensure(ctx, ctx->tmp, sizeof(T) * (size_t)ctx->nxt2 * ctx->nyt * (ctx->nz + 1));
+        return OBL_OK;
+    }
+    int fwd_prepare()
+    {
+        if (int rc = fwd_spec()) return rc;
+        return ensure(ctx, ctx->tmp, xpad_bytes());
     }
     // field c (0..3 = u, v, w, theta) of the line-kernel forward pass; its outputs d[2c],
     // d[2c+1], big[c] are final when its kernels are done
@@ -1681,6 +1695,7 @@ int obl_ctx_destroy(obl_ctx *ctx)
     cudaFree(ctx->isl_c.p);
     cudaFree(ctx->isl_d.p);
     cudaFree(ctx->tmp.p);
+    cudaFree(ctx->xpad.p);
     cudaFree(ctx->fscr.p);
     for (auto &b : ctx->rw_small) cudaFree(b.p);
     for (auto &b : ctx->rw_big) cudaFree(b.p);
