@@ -1622,11 +1622,12 @@ int obl_ctx_create(const obl_grid *grid, const obl_options *opt, obl_ctx **out)
         const size_t eb = ctx->f64 ? sizeof(double2) : sizeof(float2);
         std::vector<unsigned char> all;
         std::map<int, size_t> at;
-        for (int n : {ctx->nxt, ctx->nyt})
+        for (int n : {ctx->nxt, ctx->nyt}) {
+            if (at.count(8 * n)) continue;
+            const std::vector<std::vector<double>> tab = plan_tables(n);
             for (int role = 0; role < 2 * ROLE_TP; ++role) {
                 const int key = 8 * n + role;
-                if (at.count(key)) continue;
-                const std::vector<double> h = plan_table(n, role);
+                const std::vector<double> &h = tab[role];
                 at[key] = all.size();
                 all.resize((all.size() + eb * (h.size() / 2) + 255) / 256 * 256);
                 unsigned char *p = all.data() + at[key];
@@ -1636,6 +1637,7 @@ int obl_ctx_create(const obl_grid *grid, const obl_options *opt, obl_ctx **out)
                     for (size_t i = 0; i < h.size(); ++i) reinterpret_cast<float *>(p)[i] = (float)h[i];
                 }
             }
+        }
         if (dev_malloc(ctx, &ctx->d_tw, all.size() + 256) != cudaSuccess) return bad(OBL_ERR_NOMEM);
         for (auto &kv : at) ctx->tw[kv.first] = (unsigned char *)ctx->d_tw + kv.second;
         if (cudaMemcpy(ctx->d_tw, all.data(), all.size(), cudaMemcpyHostToDevice) != cudaSuccess) return bad(OBL_ERR_CUDA);

@@ -1054,7 +1054,7 @@ cudaError_t launch_rows_multi(int op, int n, const RowArgs<T> &a, const MultiPtr
 template <typename T>
 cudaError_t launch_cols_multi(int op, int n, const ColArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s);
 bool line_length_supported(int n);
-// twiddle table (interleaved re,im in FP64) of the plan with the given role for base length n
-std::vector<double> plan_table(int n, int role);
+// twiddle tables (interleaved re,im in FP64) of the plans of base length n, by role
+std::vector<std::vector<double>> plan_tables(int n);
 
 } // namespace obl

@@ -2,10 +2,10 @@
 #include "lines_dispatch.cuh"
 namespace obl {
 template cudaError_t launch_rows<float>(int, int, const RowArgs<float> &, cudaStream_t);
-std::vector<double> plan_table(int n, int role)
+std::vector<std::vector<double>> plan_tables(int n)
 {
     switch (n) {
-#define OBL_CASE(N) case N: return plan_table_n<N>(role);
+#define OBL_CASE(N) case N: return plan_tables_n<N>();
         OBL_FOR_EACH_N(OBL_CASE)
 #undef OBL_CASE
     }
