@@ -1,0 +1,7 @@
+// Multi-output row, column and inverse kernels of the step for double.
+#include "fused_launch.cuh"
+namespace obl {
+template struct RowsFwd3Launch<double>;
+template struct ColsFwdLaunch<double>;
+template struct PinvLaunch<double>;
+}
