@@ -628,11 +628,12 @@ enum ZOp : int { Z_UV = 0, Z_W = 1, Z_DPDZ = 2 };
 //      cst*(fun(z+1) - fun(z));
 // Z_DPDZ (103_flosol.f90:174-175): dpdz(jz) = (p(jz) - p(jz-1))/dz, jz = 1..nz-1, in slot jz-1.
 // x >= nxt is written only on the whole-plane BOGUS / zero levels.  A thread takes one
-// vector of kZLev consecutive levels (blockIdx.y; Z_DPDZ starts at level 1): kZLev + 1 loads
-// in flight for kZLev stores.  One level a thread, with the column index and both levels'
-// loads in a loop, ran at 60% of HBM: 384x384x130 levels FP32 39 -> 27 us.
-constexpr int kZLev = 8;
-template <typename T, int VW, int OP>
+// vector of ZL consecutive levels (blockIdx.y; Z_DPDZ starts at level 1): ZL + 1 loads in
+// flight for ZL stores.  Eight: one level a thread, with the column index and both levels'
+// loads in a loop, ran at 60% of HBM: 384x384x130 levels FP32 39 -> 27 us.  One below two CTAs
+// an SM, where the chain of a thread's levels counts (dpdz divides; FP64, us, eight / one:
+// 64x64x128 4.9 / 4.1, 96x96x64 6.2 / 4.1, 128x128x33 5.1 / 4.1; 128x128x64 6.1 / 6.1).
+template <typename T, int VW, int OP, int ZL>
 __global__ void __launch_bounds__(256) k_zdiff(T *__restrict__ out, const T *__restrict__ in, int nxt, int ldx,
                                                int nyt, int nz, T c)
 {
@@ -642,16 +643,16 @@ __global__ void __launch_bounds__(256) k_zdiff(T *__restrict__ out, const T *__r
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= npl) return;
     const bool inner = q % hp < ip;
-    const int z0 = blockIdx.y * kZLev + (OP == Z_DPDZ ? 1 : 0);
+    const int z0 = blockIdx.y * ZL + (OP == Z_DPDZ ? 1 : 0);
     const int lo = OP == Z_W ? z0 : z0 - 1;   // level of f[0]
     const V *vi = reinterpret_cast<const V *>(in);
     V *vo = reinterpret_cast<V *>(out);
-    V f[kZLev + 1];
+    V f[ZL + 1];
 #pragma unroll
-    for (int i = 0; i <= kZLev; ++i)   // levels past the field repeat its ends and are not used
+    for (int i = 0; i <= ZL; ++i)   // levels past the field repeat its ends and are not used
         if (inner) f[i] = vi[(long long)npl * min(max(lo + i, 0), nz) + q];
 #pragma unroll
-    for (int i = 0; i < kZLev; ++i) {
+    for (int i = 0; i < ZL; ++i) {
         const int z = z0 + i;
         V r;
         if (OP != Z_DPDZ && (z == 0 || (OP == Z_W && z == nz))) {
@@ -672,11 +673,14 @@ static void launch_zdiff(T *out, const T *in, int nxt, int ldx, int nyt, int nz,
                          cudaError_t &e)
 {
     if (e != cudaSuccess) return;
-    auto grid = [&](int vw) { return dim3((unsigned)(((ldx / vw) * nyt + 255) / 256), (unsigned)((nlev + kZLev - 1) / kZLev)); };
-    if (aligned<2>(out, in))
-        k_zdiff<T, 2, OP><<<grid(2), 256, 0, s>>>(out, in, nxt, ldx, nyt, nz, c);
-    else
-        k_zdiff<T, 1, OP><<<grid(1), 256, 0, s>>>(out, in, nxt, ldx, nyt, nz, c);
+    auto run = [&](auto vwc) {
+        constexpr int VW = decltype(vwc)::value;
+        const unsigned gx = (unsigned)(((ldx / VW) * nyt + 255) / 256), g8 = (unsigned)((nlev + 7) / 8);
+        if (gx * g8 >= 2 * 148) k_zdiff<T, VW, OP, 8><<<dim3(gx, g8), 256, 0, s>>>(out, in, nxt, ldx, nyt, nz, c);
+        else k_zdiff<T, VW, OP, 1><<<dim3(gx, (unsigned)nlev), 256, 0, s>>>(out, in, nxt, ldx, nyt, nz, c);
+    };
+    if (aligned<2>(out, in)) run(std::integral_constant<int, 2>{});
+    else run(std::integral_constant<int, 1>{});
     e = cudaGetLastError();
 }
 
