@@ -1215,30 +1215,38 @@ template <typename T> struct Ops {
         a.own_p0 = 1;
         return a;
     }
-    // Segments of the single-domain column solve (1 = whole columns).  FP32 storage: the
-    // register-segmented solve has no scratch round trip and wins from 16384 columns on
-    // (solve and RHS transforms, us, segments / whole: 192x192x128 137 / 132, 256x256x128
-    // 203 / 172, 256x256x256 374 / 282; below, 128x128x128 88 / 103).  FP64 sweeps whole
-    // columns from 49152 on (320x240x65: 263 / 225; 256x256x256 483 / 578).  Else enough
-    // segments to fill the GPU (8 resident blocks of 128 threads per SM), at least 8 levels
-    // each, a power of two (equal segments: 256x256x128 FP64 273 with 4, 307 with 5).
+    // Segments of the single-domain column solve (1 = whole columns).  Whole columns need a
+    // thread set per column and walk all levels; segments fill the GPU and pay a scratch round
+    // trip and an interface system.  The fewer levels, the more columns it takes for whole
+    // ones to win.  FP32 storage (register-segmented whole columns), step times in us with
+    // the best segments / whole: 16 levels 192x192 74 / 95, 320x384 175 / 202; 48 levels
+    // 192x192 151 / 163, 320x384 437 / 440; 65 levels 256x256 297 / 317, 320x240 385 / 398,
+    // 320x384 582 / 586; 96 levels 256x256 428 / 435, 320x240 562 / 547; 112 levels 192x160
+    // 258 / 274, 192x192 314 / 313; 256 levels 256x256 1135 / 1093.  FP64 (one thread sweeps a
+    // column): 16 levels 320x320 282 / 299; 64 levels 320x240 769 / 786, 256x384 861 / 861;
+    // 256 levels 320x240 2963 / 3023, 256x384 3310 / 3283.
+    // Segments of 8 levels where even those do not fill the GPU (8 resident blocks of 128
+    // threads per SM; 48 levels of 128x128: 87 us with 6, 92 with 4), else as many as fill it,
+    // rounded down to a power of two (256x256x128 FP64: 1234 us with 4, 1267 with 5).
     int seg_parts(long long S, int L) const
     {
         if (ctx->param_tdma_segments > 0) return (int)std::min<long long>(ctx->param_tdma_segments, L);
-        if (S >= (!ctx->f64 && ctx->param_tdma_reg && tdma_reg_supported(L) ? 16384 : 49152)) return 1;
+        const bool reg = !ctx->f64 && ctx->param_tdma_reg && tdma_reg_supported(L);
+        const long long whole = L <= 48 ? 65536 : L <= 72 || !reg ? 49152 : L <= 104 ? 36864 : 16384;
+        if (S >= whole) return 1;
         int dev = 0, nsm = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         const long long want = ((long long)nsm * 8 * 128 + S - 1) / S;
-        const long long most = std::min<long long>(std::min<long long>(want, kSlabMaxRanks), L / 8);
+        const long long most = std::max<long long>(1, std::min<long long>(kSlabMaxRanks, L / 8));
+        if (want > most) return (int)most;
         int P = 1;
-        while (2 * P <= most) P *= 2;
+        while (2 * P <= want) P *= 2;
         return P;
     }
-    // the solve's column segments for this context (with the spectral dpdz or without)
     // Segments of each FP64 island column in the mixed mode's whole-column solves (1 = the
     // island columns sweep inside the FP32 bulk launch).  The column-segmented solve serves
-    // the Neumann-top step with spectral dpdz and the three-spectra RHS.
+    // the Neumann top and the three-spectra RHS, with the spectral dpdz or without.
     int isl_parts(const TdmaArgs<T> &ta) const
     {
         if (!ctx->n_isl || ta.gform || ctx->opt.top_bc != OBL_TOP_NEUMANN) return 1;
@@ -1246,8 +1254,9 @@ template <typename T> struct Ops {
         const long long cap = std::min<long long>(kSlabMaxRanks, ctx->L / 8);
         return (int)std::max<long long>(1, std::min<long long>(P, cap));
     }
-    // (with the spectral dpdz or without: press_stag_array alone keeps whole columns, whose
-    // FP64 error is the smaller, 2e-14 against 1.6e-13 in p at 192x192x128)
+    // the solve's column segments for this context (without the spectral dpdz
+    // press_stag_array keeps whole columns, whose FP64 error is the smaller, 2e-14 against
+    // 1.6e-13 in p at 192x192x128)
     int solve_parts(bool dpdz) const
     {
         return (ctx->opt.top_bc == OBL_TOP_NEUMANN && dpdz) ? seg_parts(ctx->sp(), ctx->L) : 1;
