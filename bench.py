@@ -191,9 +191,12 @@ class Clocks:
 
 
 # ----------------------------------------------------------------------------- helpers
-def algorithmic_bytes(name, info, s):
+def algorithmic_bytes(name, info, s, launches=None, gform=False):
     """Compulsory bytes of one launch of a library kernel (its own inputs read once,
-    outputs written once); intermediates of other kernels are not counted."""
+    outputs written once); intermediates of other kernels are not counted.  launches: how
+    many launches of a step carry the name (the four fields' rows_fwd3 are one launch where
+    the forward pass is batched, four where it runs field by field); gform: the step forms
+    the pressure RHS in G form, whose H_x and H_z are not y-transformed with H_y."""
     nx, ny, nz = info["nxt"], info["nyt"], info["nz"]
     nx2, ny2, lhx = info["nxt2"], info["nyt2"], info["lhx"]
     L, nlev = nz - 1, nz + 1
@@ -211,9 +214,16 @@ def algorithmic_bytes(name, info, s):
         "tdma_staged": 5 * lhx * ny * L * c,
         # levels 1..L of H_x and 0..L+1 of H_z in, the y-transform of G over H_x out (2 launches)
         "press_gform_cols": ((L + (L + 2) + L) * lhx * ny * c) / 2,
-        # one launch per field: field in, ddx and the x-padded rows out, and on u, v, w the
-        # RHS x-spectrum of levels 1..L out (mean over the 4 launches of a step)
-        "rows_fwd3": ((2 * nx + nx2) * ny * nlev * s * 4 + 3 * lhx * ny * L * c) / 4,
+        # four fields in, ddx and the x-padded rows out, and of u, v, w the RHS x-spectrum of
+        # levels 1..L out
+        "rows_fwd3": ((2 * nx + nx2) * ny * nlev * s * 4 + 3 * lhx * ny * L * c) / (launches or 4),
+        # the column work of the batched forward pass: y-pad and ddy of four fields, y-transform
+        # of the RHS spectra
+        "cols_fwd": ((nx2 * ny + nx2 * ny2) + 2 * nx * ny) * nlev * s * 4 + (1 if gform else 3) * 2 * lhx * ny * L * c,
+        # segmented columns: three RHS spectra in, y' and the real v', c' of levels 1..L out;
+        # those in, p_hat and the dpdz spectrum out
+        "tdma_seg_solve": 5 * lhx * ny * L * c,
+        "tdma_seg_finish": 4 * lhx * ny * L * c,
         # p_hat (0..L) and the dpdz spectrum in; y-inverses of p, dpdy, dpdz out (dpdx's is
         # i*kx times that of p, formed by the row pass)
         "pinv_cols": (2 * L + 1) * lhx * ny * c + (3 * L + 1) * lhx * ny * c,
@@ -368,7 +378,7 @@ def run_ours(args, rank, local, world):
     ctx.timing(False)
     dom = max(kt.items(), key=lambda kv: kv[1][1])
     dom_name, (dom_n, dom_ms) = dom[0], dom[1]
-    ab = algorithmic_bytes(dom_name, ctx.info, es)
+    ab = algorithmic_bytes(dom_name, ctx.info, es, dom_n, "press_gform_cols" in kt)
     traffic = None
     try:
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as fh:
