@@ -76,7 +76,10 @@ int ens_lines_of(int n);   // lines per unit of an instance's line transforms of
 // y-inverse), <4,6,2> (x-inverse + project).  FP64 butterflies need the registers of 2 CTAs
 // per SM (bounded for 4, the 48-instance step took 44.6 instead of 36.4 ms in the split form).
 #ifndef OBL_ENS_MINB
-#define OBL_ENS_MINB 4   // CTAs per SM the FP32 one-launch persistent kernel's registers are bounded for
+// CTAs per SM the FP32 one-launch persistent kernel's registers are bounded for (ms of the
+// 48-instance step, grid barriers / dataflow: 4 19.1 / 26.1, 3 18.7 / 27.1, 2 27.7 / 29.4;
+// eight 64x64x32 instances 0.278 / 0.269, 0.288 / 0.284, 0.319 / 0.324)
+#define OBL_ENS_MINB 4
 #endif
 template <typename T> constexpr int ens_minb() { return sizeof(T) == 8 ? 2 : OBL_ENS_MINB; }
 template <typename T> constexpr int ens_minb_mid() { return sizeof(T) == 8 ? 2 : 4; }

@@ -102,7 +102,7 @@ BUILD_CANDIDATES = {
     "cols_4w4l": ["OBL_TP_LINES=4"],
     "cols_16w_sm": ["OBL_TP_WARPS_SM=16"],
     "cols_32w_sm": ["OBL_TP_WARPS_SM=32"],
-    "rows_pad16": ["OBL_SIDX_SHIFT=4"],
+    "rows_pad16": ["OBL_SIDX_SHIFT=4"],   # the cluster-fused plane kernels ("fused" = 1)
     "pad_prefetch_off": ["OBL_COL_PF=0"],
 }
 
