@@ -7,8 +7,8 @@ namespace obl {
 constexpr int kFillPer = 4096;   // elements of a BOGUS plane per CTA
 
 // ddx of WB row pairs by two passes, the other terms added at the store.  The addends are
-// asked into L2 when the unit starts and read in groups of eight elements a row, so that a
-// group's loads (up to 48) are in flight together.
+// asked into L2 when the unit starts and read in groups of four elements a row, so that a
+// group's loads (up to 24) are in flight together.
 template <typename T, int N>
 __global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb)
     k_tp_rows_divt(RowArgs<T> a, const __grid_constant__ DivRows<T> e, int nb, int nfill)

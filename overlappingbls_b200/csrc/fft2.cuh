@@ -229,11 +229,4 @@ template <int N, int R, int LL> struct Geo {
     static constexpr bool FULL = (NB % LL) == 0;
 };
 
-// Host-side twiddle table of a plan (same layout as the device blocks).
-template <class P> struct PlanList;
-template <int... Rs> struct PlanList<RPlan<Rs...>> {
-    static constexpr int n = sizeof...(Rs);
-    static constexpr int r[sizeof...(Rs)] = {Rs...};
-};
-
 } // namespace obl

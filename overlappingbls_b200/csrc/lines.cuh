@@ -10,10 +10,10 @@
 // per-line r2c -> op -> c2r computes (004_derivatives.f90:33-39,
 // 108_01_padd.f90:102-127,163-190).
 //
-// Rows are loaded from global memory straight into registers in the layout of the
-// first FFT pass; columns are staged through a shared-memory tile (the on-GPU
-// replacement of the reference's mpi_alltoall pencil transposes,
-// 203_fftn_mpi.f90:71-371) whose padded column doubles as the FFT exchange scratch.
+// Rows and columns are loaded from global memory straight into registers in the layout of
+// the first FFT pass and exchanged through shared memory; a column CTA's WB adjacent lines
+// make its accesses row segments (the on-GPU replacement of the reference's mpi_alltoall
+// pencil transposes, 203_fftn_mpi.f90:71-371).
 //
 // Accuracy: before a real line is transformed, its first value is subtracted (exact
 // by Sterbenz's lemma for fields with a large mean such as theta ~ 300 K) and the
@@ -60,9 +60,8 @@ template <typename T> struct ColArgs {
     const C2<T> *twF, *twB;
     int pad_copy;                    // UNPAD: also write columns 0,1 into ncols, ncols+1
     int zero_nyq;                    // FWD: zero the Nyquist row (203_fftn_mpi.f90:33)
-    int pf_ahead;                    // the unit of plane z also prefetches its input lines of
-                                     // plane z + pf_ahead into L2 (0 = none)
     int tma;                         // FP32 y-pad: input tile by tensor-map copies (k_tp_cols_tma)
+    int pf_ahead;                    // those also ask L2 for the tile of plane z + pf_ahead (0 = none)
     int *wait_err;                   // set to 1 when such a copy's bounded wait gave up
 };
 
@@ -77,11 +76,6 @@ template <int N> struct LineCfg<N, OP_PAD> {
     static constexpr int NI = N, NO = 3 * N / 2;
     using PF = FwdPlan<N>;
     using PB = PadBwdPlan<N>;
-};
-template <int N> struct LineCfg<N, OP_UNPAD> {
-    static constexpr int NI = 3 * N / 2, NO = N;
-    using PF = PadFwdPlan<N>;
-    using PB = BwdPlan<N>;
 };
 template <int N> struct LineCfg<N, OP_FWD> : LineCfg<N, OP_DERIV> {};
 template <int N> struct LineCfg<N, OP_INV> : LineCfg<N, OP_DERIV> {};
@@ -140,36 +134,6 @@ __device__ __forceinline__ void reg_pad(const C2<T> *v, C2<T> *w, int t)
             w[b * R2 + r2] = x;
         }
     }
-}
-
-// D(3R/2) of length 3N/2  ->  D(R) of length N, truncated, new Nyquist bin zero
-template <typename T, int N, int R, int LL>
-__device__ __forceinline__ void reg_unpad(const C2<T> *w, C2<T> *v, int t)
-{
-    using G = Geo<N, R, LL>;
-    constexpr int R2 = 3 * R / 2, H = R / 2;
-#pragma unroll
-    for (int b = 0; b < G::PER; ++b) {
-        const int j = t + LL * b;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            C2<T> x = (r < H) ? w[b * R2 + r] : w[b * R2 + r + H];
-            if (r == H && j == 0) x = mk<T>(0, 0);     // bin N/2
-            v[b * R + r] = x;
-        }
-    }
-}
-
-// ----------------------------------------------------------------------------- row kernel
-// copy the plan twiddle tables an op needs into shared memory (caller syncs)
-template <typename T, int N, int OP>
-__device__ __forceinline__ void load_tables(const C2<T> *gF, const C2<T> *gB, C2<T> *sF, C2<T> *sB)
-{
-    using D = LineDerived<N, OP>;
-    if (OP != OP_INV)
-        for (int i = threadIdx.x; i < D::TF; i += blockDim.x) sF[i] = gF[i];
-    if (OP != OP_FWD)
-        for (int i = threadIdx.x; i < D::TB; i += blockDim.x) sB[i] = gB[i];
 }
 
 // ----------------------------------------------------------------------------- column kernel
@@ -236,7 +200,7 @@ __device__ __forceinline__ void col_unit(const ColArgs<T> &a, int z, int tx, con
     C v[VR];
     T cr = 0, ci = 0;
 
-    static_assert(OP != OP_INV, "forward passes only");
+    static_assert(OP == OP_DERIV || OP == OP_PAD || OP == OP_FWD, "the passes of the cluster-fused kernel");
     auto body = [&](auto &acc) {
         {
             using G = Geo<NI, D::RF0, LL>;
@@ -281,11 +245,10 @@ __device__ __forceinline__ void col_unit(const ColArgs<T> &a, int z, int tx, con
             C *vb = v;
             if constexpr (OP == OP_DERIV) reg_deriv<T, N, D::RFL, LL>(v, a.ktab, t);
             if constexpr (OP == OP_PAD) { reg_pad<T, N, D::RFL, LL>(v, w, t); vb = w; }
-            if constexpr (OP == OP_UNPAD) { reg_unpad<T, N, D::RB0, LL>(v, w, t); vb = w; }
             fft_regs<NO, typename D::PB, LL, false>(vb, acc, twB, t);
             using G = Geo<NO, D::RBL, LL>;
-            const T ar = (OP == OP_PAD || OP == OP_UNPAD) ? cr : (T)0;
-            const T ai = (OP == OP_PAD || OP == OP_UNPAD) ? ci : (T)0;
+            const T ar = OP == OP_PAD ? cr : (T)0;
+            const T ai = OP == OP_PAD ? ci : (T)0;
 #pragma unroll
             for (int b = 0; b < G::PER; ++b) {
                 const int j = t + LL * b;
@@ -312,15 +275,6 @@ __device__ __forceinline__ void col_unit(const ColArgs<T> &a, int z, int tx, con
     for (int idx = threadIdx.x; idx < NO * W; idx += blockDim.x) {
         const int r = idx / W, cx = idx - r * W;
         if (cx < nc) dst[(long long)r * a.dst_row + cx] = tile[sidx(r) * S + cx];
-    }
-    if constexpr (OP == OP_UNPAD && REAL) {
-        // var(nxt+1:ldx,:) = var(1:2,:) (108_01_padd.f90:195)
-        if (a.pad_copy && c0 == 0)
-            for (int r = threadIdx.x; r < NO; r += blockDim.x) {
-                E *d = reinterpret_cast<E *>(a.dst) + (long long)z * a.dst_plane + (long long)r * a.dst_row;
-                d[a.ncols] = tile[sidx(r) * S + 0];
-                d[a.ncols + 1] = tile[sidx(r) * S + 1];
-            }
     }
     __syncthreads();   // the tile may be reused by the caller's next unit
 }
@@ -472,7 +426,7 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
                 for (int r = 0; r < RI; ++r) v[b][r] = x[r];
             }
         }
-        if constexpr (OP != OP_FWD) __syncthreads();   // the exchange is read before it is written again
+        __syncthreads();   // the exchange is read before it is written again
     } else {
 #pragma unroll
         for (int b = 0; b < PER2; ++b) {
@@ -485,61 +439,45 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
             }
         }
     }
-    if constexpr (OP == OP_FWD) {
+#pragma unroll
+    for (int b = 0; b < PER2; ++b) {
+        const int j = (tid + b * NT) / WB;
+        if constexpr (OP == OP_PAD) {
+            if (j == 0) v[b][RI / 2] = mk<T>(0, 0);   // the source's Nyquist bin
+            DftPad<D::R1>::run(v[b], [&](auto ic, C x) { buf[(j * D::PO + decltype(ic)::value) * WB + line] = x; });
+        } else {
+            if constexpr (OP == OP_DERIV) tp_deriv<T, N, R0, RO>(v[b], a.ktab, j);
+            if constexpr (OP == OP_FILT) if (j == 0) v[b][RO / 2] = mk<T>(0, 0);
+            Dft<RO, false>::run(v[b]);
+#pragma unroll
+            for (int r = 0; r < RO; ++r) buf[(j * D::PO + r) * WB + line] = v[b][r];
+        }
+    }
+    __syncthreads();
+    constexpr bool addc = OP == OP_PAD || OP == OP_UNPAD;
+#pragma unroll 1
+    for (int f = tid; f < I3; f += NT) {
+        const int j = f / WB;
+        C x[R0];
+#pragma unroll
+        for (int r = 0; r < R0; ++r) x[r] = buf[(r * D::PO + j) * WB + line];
+#pragma unroll
+        for (int r = 1; r < R0; ++r) x[r] = cmulc(x[r], __ldg(a.twB + r * RO + j));
+        Dft<R0, false>::run(x);
         if (act) {
 #pragma unroll
-            for (int b = 0; b < PER2; ++b) {
-                const int j = (tid + b * NT) / WB;
-#pragma unroll
-                for (int r = 0; r < RI; ++r) {
-                    const int i = j + r * R0;
-                    C x = v[b][r];
-                    if (r == RI / 2 && a.zero_nyq && j == 0) x = mk<T>(0, 0);   // bin N/2
-                    gst(i, x);
+            for (int r = 0; r < R0; ++r) {
+                const int i = j + r * RO;
+                C y = x[r];
+                if (addc) {
+                    y.x += cref.x;
+                    y.y += cref.y;
                 }
-            }
-        }
-    } else {
-#pragma unroll
-        for (int b = 0; b < PER2; ++b) {
-            const int j = (tid + b * NT) / WB;
-            if constexpr (OP == OP_PAD) {
-                if (j == 0) v[b][RI / 2] = mk<T>(0, 0);   // the source's Nyquist bin
-                DftPad<D::R1>::run(v[b], [&](auto ic, C x) { buf[(j * D::PO + decltype(ic)::value) * WB + line] = x; });
-            } else {
-                if constexpr (OP == OP_DERIV) tp_deriv<T, N, R0, RO>(v[b], a.ktab, j);
-                if constexpr (OP == OP_FILT) if (j == 0) v[b][RO / 2] = mk<T>(0, 0);
-                Dft<RO, false>::run(v[b]);
-#pragma unroll
-                for (int r = 0; r < RO; ++r) buf[(j * D::PO + r) * WB + line] = v[b][r];
-            }
-        }
-        __syncthreads();
-        constexpr bool addc = OP == OP_PAD || OP == OP_UNPAD;
-#pragma unroll 1
-        for (int f = tid; f < I3; f += NT) {
-            const int j = f / WB;
-            C x[R0];
-#pragma unroll
-            for (int r = 0; r < R0; ++r) x[r] = buf[(r * D::PO + j) * WB + line];
-#pragma unroll
-            for (int r = 1; r < R0; ++r) x[r] = cmulc(x[r], __ldg(a.twB + r * RO + j));
-            Dft<R0, false>::run(x);
-            if (act) {
-#pragma unroll
-                for (int r = 0; r < R0; ++r) {
-                    const int i = j + r * RO;
-                    C y = x[r];
-                    if (addc) {
-                        y.x += cref.x;
-                        y.y += cref.y;
-                    }
-                    gst(i, y);
-                    if constexpr (OP == OP_UNPAD && REAL) {
-                        // var(nxt+1:ldx,:) = var(1:2,:) (108_01_padd.f90:195)
-                        if (a.pad_copy && gl == 0 && ck_in(a.ncols + 1, a.dst_row, CK_COL_STORE))
-                            *reinterpret_cast<C *>(dstz + (long long)i * a.dst_row + a.ncols) = y;
-                    }
+                gst(i, y);
+                if constexpr (OP == OP_UNPAD && REAL) {
+                    // var(nxt+1:ldx,:) = var(1:2,:) (108_01_padd.f90:195)
+                    if (a.pad_copy && gl == 0 && ck_in(a.ncols + 1, a.dst_row, CK_COL_STORE))
+                        *reinterpret_cast<C *>(dstz + (long long)i * a.dst_row + a.ncols) = y;
                 }
             }
         }
@@ -549,7 +487,7 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
 // Threads, lines and registers of the column kernels: WB lines (64-byte row segments; 128
 // bytes for the short lines of R0 = 8), R0*WB/PER2 threads.  FP32: 24 resident warps with
 // one middle butterfly a thread (80 registers) beat 16 warps with two (y-pad of 512 lines,
-// 258 levels: 0.846 against 0.881 ms over four fields; 20 warps spill: 0.949), except
+// 258 levels, as first built: 0.846 against 0.881 ms over four fields; 20 warps spill: 0.949), except
 // where all threads load at once in the forward-only transform (0.351 against 0.388 ms for
 // three spectra).  FP64 radix-32 butterflies need 8 warps; two middle butterflies a thread
 // keep more of them loading (ddy 1.214 against 1.450 ms), which the y-pad's larger exchange
@@ -558,7 +496,7 @@ __device__ __forceinline__ void tp_cols_unit(const ColArgs<T> &a, int bx, int z,
 // y-pad 1.243 -> 0.888, ddy 0.714 -> 0.566, y-transform 0.393 -> 0.358; FP64 y-pad 3.00 ->
 // 2.31, ddy 1.85 -> 1.30; at 128x128 levels the y-pad takes 0.62 and the y-unpad 0.55 of
 // their time.
-// The L1/shared pipe fell from 70 to 55% busy at half the time per byte.  A persistent form
+// The L1/shared pipe fell from 69 to 55% busy (y-pad of 64 levels, 91 -> 66 us).  A persistent form
 // with the next tile's copies in flight measured slower (1.25 ms): its second tile leaves
 // shared memory for 16 warps only.
 #ifndef OBL_TP_WARPS_SM
