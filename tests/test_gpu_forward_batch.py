@@ -1,11 +1,17 @@
 """GPU tests of the device step's batched forward pass (all four fields' rows, then columns,
-in two launches) and of the memory it takes."""
+in two launches) and of the memory it takes: every line length once along x and once along
+y, with partial CTAs, with and without surface planes, in G form (FP64, whole columns) and
+not, against the oracle; both sides of its 512 MB line; and the same under index checks."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import overlappingbls_b200 as obl
-from overlappingbls_b200 import fields
-from conftest import identical_inputs, rel_l2
+from overlappingbls_b200 import build, fields
+from conftest import ROOT, identical_inputs, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -69,6 +75,52 @@ def _launches(ctx, call):
     names = {k: v[0] for k, v in ctx.timing_report().items()}
     ctx.timing(False)
     return names
+
+
+LENGTHS = (32, 48, 64, 80, 96, 128, 160, 192, 240, 256, 320, 384, 512, 640)
+
+
+@pytest.mark.parametrize("prec", ["f64", "mixed"])
+@pytest.mark.parametrize("i,nx", list(enumerate(LENGTHS)))
+def test_batched_step_every_length(orc, i, nx, prec):
+    ny = LENGTHS[(i + 5) % len(LENGTHS)]
+    ctx, g, f = _setup(orc, nx, ny, 10, prec)      # 9 levels: whole columns
+    planes = {}
+    if i % 2:
+        planes = {k: np.asfortranarray((1e-3 * f[v][:, :, 2]).astype(np.float32).astype(np.float64))
+                  for k, v in (("bot", "v"), ("top", "w"))}
+    s = DevStep(ctx, f, prec, planes)
+    names = _launches(ctx, s.run)
+    assert names["rows_fwd3"] == 1 and names["cols_fwd"] == 1 and "pad_cols" not in names, names
+    assert ("press_gform_cols" in names) == (prec == "f64"), names
+    ref = g.step(f["u"], f["v"], f["w"], f["theta"], npz=3)
+    if planes:
+        p, dx, dy = g.press_stag_array(f["u"], f["v"], f["w"], planes["bot"], planes["top"], npz=3)
+        dz = g.dpdz(p)
+        ref.update(p=p, dpdx=dx, dpdy=dy, dpdz=dz, **dict(zip("uvw", g.project(f["u"], f["v"], f["w"], dx, dy, dz))))
+    s.check(ref, TOL[prec])
+    ctx.close()
+
+
+# 4 fields of 960 x 640 x nlev doubles: 530.8 MB at 27 stored levels, 550.5 MB at 28 (limit 536.9)
+@pytest.mark.parametrize("nzt,batched", [(26, True), (27, False)])
+def test_both_sides_of_the_memory_line(orc, nzt, batched):
+    ctx, g, f = _setup(orc, 640, 640, nzt, "f64")
+    s = DevStep(ctx, f, "f64")
+    names = _launches(ctx, s.run)
+    assert ("cols_fwd" in names) == batched and ("pad_cols" in names) != batched, names
+    s.check(g.step(f["u"], f["v"], f["w"], f["theta"], npz=5 if nzt == 26 else 2), TOL["f64"])
+    ctx.close()
+
+
+def test_batched_step_under_index_checks():
+    if os.environ.get("OBL_CHECKED_RUN") == "1":
+        pytest.skip("already the child run")
+    env = dict(os.environ, OBL_LIB=build.LIB_CHECK, OBL_CHECKED_RUN="1")
+    r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-p", "no:cacheprovider", __file__, "-k", "every_length"],
+                       cwd=ROOT, env=env, capture_output=True, text=True, timeout=1200)
+    tail = "\n".join(r.stdout.splitlines()[-25:])
+    assert r.returncode == 0 and "28 passed" in tail, tail
 
 
 def test_step_without_memory_for_the_batch(orc):
