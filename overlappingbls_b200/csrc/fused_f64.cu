@@ -1,7 +1,6 @@
-// Multi-output row, column and inverse kernels of the step for double.
+// Multi-output row and column kernels of the step for double.
 #include "fused_launch.cuh"
 namespace obl {
 template struct RowsFwd3Launch<double>;
 template struct ColsFwdLaunch<double>;
-template struct PinvLaunch<double>;
 }

@@ -1,7 +1,5 @@
-// fused_launch.cuh -- launchers of the step's multi-output kernels (fused.cuh), one unit of
-// compilation per precision (fused_f32.cu, fused_f64.cu): a process loads what the first call
-// into a unit brings with it, and loading both precisions and the cluster-fused kernels
-// together made the first step 63 ms where one precision's takes XX.
+// fused_launch.cuh -- launchers of the step's multi-output kernels (fused.cuh), in units of
+// compilation by precision (fused_*.cu, pinv_*.cu; see launch_cols in lines.cuh).
 #pragma once
 #include "fused.cuh"
 #include "lines_dispatch.cuh"

@@ -976,7 +976,17 @@ template <typename T, int N, int OP, bool REAL> cudaError_t launch_cols_t(const 
 
 // Runtime dispatch: n is the base length (the unpadded one for PAD/UNPAD).
 template <typename T> cudaError_t launch_rows(int op, int n, const RowArgs<T> &a, cudaStream_t s);
-template <typename T> cudaError_t launch_cols(int op, bool real, int n, const ColArgs<T> &a, cudaStream_t s);
+// (The kernels behind them are spread over units of compilation by precision and kind: the
+// first call into a unit loads all of it, and nvcc compresses a large one.  The first FP64 ddy
+// of a process took 10.8 ms with the complex columns in the same unit, 3.0 without; the first
+// press_stag_array 59 to 100 ms with the multi-field, step and inverse kernels of both
+// precisions in two units, 12 in units of their own; the first step 49 and 16 ms.)
+template <typename T> cudaError_t launch_cols_real(int op, int n, const ColArgs<T> &a, cudaStream_t s);
+template <typename T> cudaError_t launch_cols_cplx(int op, int n, const ColArgs<T> &a, cudaStream_t s);
+template <typename T> inline cudaError_t launch_cols(int op, bool real, int n, const ColArgs<T> &a, cudaStream_t s)
+{
+    return real ? launch_cols_real<T>(op, n, a, s) : launch_cols_cplx<T>(op, n, a, s);
+}
 
 // The same line ops on up to kMultiFields fields of one shape in one launch: field f
 // reads src[f] and writes dst[f]; the args' src/dst are ignored.  Rows: OP_DERIV, OP_PAD,
@@ -988,9 +998,25 @@ template <typename T> struct MultiPtr {
     void *dst[kMultiFields];
 };
 template <typename T>
-cudaError_t launch_rows_multi(int op, int n, const RowArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s);
+cudaError_t launch_rows_multi_fwd(int n, const RowArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s);
 template <typename T>
-cudaError_t launch_cols_multi(int op, int n, const ColArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s);
+cudaError_t launch_cols_multi_fwd(int n, const ColArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s);
+template <typename T>
+cudaError_t launch_rows_multi_real(int op, int n, const RowArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s);
+template <typename T>
+cudaError_t launch_cols_multi_real(int op, int n, const ColArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s);
+template <typename T>
+inline cudaError_t launch_rows_multi(int op, int n, const RowArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
+{
+    if (nf < 1 || nf > kMultiFields) return cudaErrorInvalidValue;
+    return op == OP_FWD ? launch_rows_multi_fwd<T>(n, a, m, nf, s) : launch_rows_multi_real<T>(op, n, a, m, nf, s);
+}
+template <typename T>
+inline cudaError_t launch_cols_multi(int op, int n, const ColArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
+{
+    if (nf < 1 || nf > kMultiFields) return cudaErrorInvalidValue;
+    return op == OP_FWD ? launch_cols_multi_fwd<T>(n, a, m, nf, s) : launch_cols_multi_real<T>(op, n, a, m, nf, s);
+}
 bool line_length_supported(int n);
 // twiddle tables (interleaved re,im in FP64) of the plans of base length n, by role
 std::vector<std::vector<double>> plan_tables(int n);

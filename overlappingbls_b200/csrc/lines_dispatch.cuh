@@ -26,20 +26,22 @@ cudaError_t rows_n(int op, const RowArgs<T> &a, cudaStream_t s)
 }
 
 template <typename T, int N>
-cudaError_t cols_n(int op, bool real, const ColArgs<T> &a, cudaStream_t s)
+cudaError_t cols_real_n(int op, const ColArgs<T> &a, cudaStream_t s)
 {
-    if (real) {
-        switch (op) {
-        case OP_DERIV: return launch_cols_t<T, N, OP_DERIV, true>(a, s);
-        case OP_PAD: return launch_cols_t<T, N, OP_PAD, true>(a, s);
-        case OP_UNPAD: return launch_cols_t<T, N, OP_UNPAD, true>(a, s);
-        }
-    } else {
-        switch (op) {
-        case OP_FWD: return launch_cols_t<T, N, OP_FWD, false>(a, s);
-        case OP_INV: return launch_cols_t<T, N, OP_INV, false>(a, s);
-        case OP_FILT: return launch_cols_t<T, N, OP_FILT, false>(a, s);
-        }
+    switch (op) {
+    case OP_DERIV: return launch_cols_t<T, N, OP_DERIV, true>(a, s);
+    case OP_PAD: return launch_cols_t<T, N, OP_PAD, true>(a, s);
+    case OP_UNPAD: return launch_cols_t<T, N, OP_UNPAD, true>(a, s);
+    }
+    return cudaErrorInvalidValue;
+}
+template <typename T, int N>
+cudaError_t cols_cplx_n(int op, const ColArgs<T> &a, cudaStream_t s)
+{
+    switch (op) {
+    case OP_FWD: return launch_cols_t<T, N, OP_FWD, false>(a, s);
+    case OP_INV: return launch_cols_t<T, N, OP_INV, false>(a, s);
+    case OP_FILT: return launch_cols_t<T, N, OP_FILT, false>(a, s);
     }
     return cudaErrorInvalidValue;
 }
@@ -54,10 +56,19 @@ template <typename T> cudaError_t launch_rows(int op, int n, const RowArgs<T> &a
     return cudaErrorInvalidValue;
 }
 
-template <typename T> cudaError_t launch_cols(int op, bool real, int n, const ColArgs<T> &a, cudaStream_t s)
+template <typename T> cudaError_t launch_cols_real(int op, int n, const ColArgs<T> &a, cudaStream_t s)
 {
     switch (n) {
-#define OBL_CASE(N) case N: return cols_n<T, N>(op, real, a, s);
+#define OBL_CASE(N) case N: return cols_real_n<T, N>(op, a, s);
+        OBL_FOR_EACH_N(OBL_CASE)
+#undef OBL_CASE
+    }
+    return cudaErrorInvalidValue;
+}
+template <typename T> cudaError_t launch_cols_cplx(int op, int n, const ColArgs<T> &a, cudaStream_t s)
+{
+    switch (n) {
+#define OBL_CASE(N) case N: return cols_cplx_n<T, N>(op, a, s);
         OBL_FOR_EACH_N(OBL_CASE)
 #undef OBL_CASE
     }

@@ -1,6 +1,7 @@
-// multi.cu -- the row and column line kernels over several fields of one shape in one
+// multi.cuh -- the row and column line kernels over several fields of one shape in one
 // launch (see launch_rows_multi / launch_cols_multi in lines.cuh).  The per-line work is
 // tp_row_unit / tp_cols_unit unchanged; only the field of each unit is looked up first.
+#pragma once
 #include "lines_dispatch.cuh"
 
 namespace obl {
@@ -78,7 +79,6 @@ static cudaError_t rows_multi_n(int op, const RowArgs<T> &a, const MultiPtr<T> &
     case OP_DERIV: return rows_multi_t<T, N, OP_DERIV>(a, m, nf, s);
     case OP_PAD: return rows_multi_t<T, N, OP_PAD>(a, m, nf, s);
     case OP_UNPAD: return rows_multi_t<T, N, OP_UNPAD>(a, m, nf, s);
-    case OP_FWD: return rows_multi_t<T, N, OP_FWD>(a, m, nf, s);
     }
     return cudaErrorInvalidValue;
 }
@@ -90,15 +90,13 @@ static cudaError_t cols_multi_n(int op, const ColArgs<T> &a, const MultiPtr<T> &
     case OP_DERIV: return cols_multi_t<T, N, OP_DERIV, true>(a, m, nf, s);
     case OP_PAD: return cols_multi_t<T, N, OP_PAD, true>(a, m, nf, s);
     case OP_UNPAD: return cols_multi_t<T, N, OP_UNPAD, true>(a, m, nf, s);
-    case OP_FWD: return cols_multi_t<T, N, OP_FWD, false>(a, m, nf, s);   // complex columns
     }
     return cudaErrorInvalidValue;
 }
 
 template <typename T>
-cudaError_t launch_rows_multi(int op, int n, const RowArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
+cudaError_t launch_rows_multi_real(int op, int n, const RowArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
 {
-    if (nf < 1 || nf > kMultiFields) return cudaErrorInvalidValue;
     switch (n) {
 #define OBL_CASE(N) case N: return rows_multi_n<T, N>(op, a, m, nf, s);
         OBL_FOR_EACH_N(OBL_CASE)
@@ -108,9 +106,8 @@ cudaError_t launch_rows_multi(int op, int n, const RowArgs<T> &a, const MultiPtr
 }
 
 template <typename T>
-cudaError_t launch_cols_multi(int op, int n, const ColArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
+cudaError_t launch_cols_multi_real(int op, int n, const ColArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
 {
-    if (nf < 1 || nf > kMultiFields) return cudaErrorInvalidValue;
     switch (n) {
 #define OBL_CASE(N) case N: return cols_multi_n<T, N>(op, a, m, nf, s);
         OBL_FOR_EACH_N(OBL_CASE)
@@ -119,13 +116,27 @@ cudaError_t launch_cols_multi(int op, int n, const ColArgs<T> &a, const MultiPtr
     return cudaErrorInvalidValue;
 }
 
-template cudaError_t launch_rows_multi<float>(int, int, const RowArgs<float> &, const MultiPtr<float> &, int,
-                                              cudaStream_t);
-template cudaError_t launch_rows_multi<double>(int, int, const RowArgs<double> &, const MultiPtr<double> &, int,
-                                               cudaStream_t);
-template cudaError_t launch_cols_multi<float>(int, int, const ColArgs<float> &, const MultiPtr<float> &, int,
-                                              cudaStream_t);
-template cudaError_t launch_cols_multi<double>(int, int, const ColArgs<double> &, const MultiPtr<double> &, int,
-                                               cudaStream_t);
+template <typename T>
+cudaError_t launch_rows_multi_fwd(int n, const RowArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
+{
+    switch (n) {
+#define OBL_CASE(N) case N: return rows_multi_t<T, N, OP_FWD>(a, m, nf, s);
+        OBL_FOR_EACH_N(OBL_CASE)
+#undef OBL_CASE
+    }
+    return cudaErrorInvalidValue;
+}
+
+// (complex columns)
+template <typename T>
+cudaError_t launch_cols_multi_fwd(int n, const ColArgs<T> &a, const MultiPtr<T> &m, int nf, cudaStream_t s)
+{
+    switch (n) {
+#define OBL_CASE(N) case N: return cols_multi_t<T, N, OP_FWD, false>(a, m, nf, s);
+        OBL_FOR_EACH_N(OBL_CASE)
+#undef OBL_CASE
+    }
+    return cudaErrorInvalidValue;
+}
 
 } // namespace obl
