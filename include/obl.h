@@ -103,9 +103,10 @@ int obl_timing_report(obl_ctx *ctx, char *buf, size_t n);
      "fwd_clusters"      clusters of the fused forward kernel (0 = as many as can be resident)
      "fwd_cluster_size"  CTAs per cluster (1..16; above 8 needs non-portable cluster support)
      "tdma_segments"     segments each (kx,ky) column of the pressure solve is split into
-                         and solved at once (0 = chosen by size: more than one only when
-                         the columns alone cannot fill the GPU; 1 = one sequential sweep;
-                         up to 16; used in the Neumann-top mode with spectral dpdz)
+                         and solved at once (0 = chosen by the columns and levels: more than
+                         one below 65536 columns, and from 49 levels on below 49152, with
+                         FP32 storage 36864 from 73 levels and 16384 from 105; 1 = whole
+                         columns; up to 16; used in the Neumann-top mode with spectral dpdz)
      "tdma_reg"          FP32 storage: 1 = the register-segmented whole-column solve
                          (default), 0 = one sequential sweep per column
      "tdma_stage"        with "tdma_reg": 1 = its persistent form fed by bulk asynchronous
@@ -120,9 +121,12 @@ int obl_timing_report(obl_ctx *ctx, char *buf, size_t n);
                          (default 0: measured slower)
      "gform"             the pressure RHS in G form: 1 = with FP64 storage (default),
                          2 = always, 0 = never
-     "pad_tma"           FP32 y-pad (zero_padding, the step): 1 = each CTA's input tile by
+     "pad_tma"           FP32 y-pad of lines from 256 on (zero_padding, and the step where its
+                         forward pass runs field by field): 1 = each CTA's input tile by
                          tensor-map copies (default), 0 = by loads
-     "fwd_chunk"         the step's forward pass over chunks of this many levels (0 = all)
+     "fwd_chunk"         n > 0: the device step's forward pass field by field over chunks of
+                         n levels; 0 = all levels at once, and the four fields in two
+                         launches where their x-padded intermediates take up to 512 MB
      "out_streams"       copy streams of the host-array step's outputs (1 or 2; default 2)
      "fail_alloc"        n > 0: the n-th device allocation from now fails (tests)
      "stage_timeout_test" 1: the staged solve's waits expect bytes no copy delivers, so
@@ -238,7 +242,9 @@ int obl_filter_data_dev(obl_ctx *ctx, void *f, int nlev);
    u,v,w (ldx,nyt,0:nz) in; divtz_bot = divtz(:,:,1), divtz_top = divtz(:,:,nz)
    planes (ldx,nyt) or NULL for zero (the theta/lbc==0 surface term of :187-192 is
    folded into divtz_bot by the caller); p (ldx,nyt,0:nz) levels 0..nz-1 written;
-   dpdx, dpdy (ldx,nyt,1:nz) levels 1..nz-1 written. */
+   dpdx, dpdy (ldx,nyt,1:nz) levels 1..nz-1 written.  With FP32 storage the host variant's
+   transforms are the three-radix ones, so that its real(8) results do not change with the
+   factorisation the device variants use (both are as exact). */
 int obl_press_stag_array(obl_ctx *ctx, const double *u, const double *v, const double *w,
                          const double *divtz_bot, const double *divtz_top,
                          double *p, double *dpdx, double *dpdy);
@@ -261,7 +267,11 @@ int obl_project_dev(obl_ctx *ctx, void *u, void *v, void *w,
    u,v,w,theta and zero_padding of u,v,w,theta on levels 0..nz (103_flosol.f90:30-35,
    108_convec.f90:38-42, 010_scalars.f90:137-138,429-431), press_stag_array(u,v,w),
    dpdz and project (103_flosol.f90:168-188).  Pointers are host (obl_step /
-   obl_step_f32) or device (obl_step_dev, storage type). */
+   obl_step_f32) or device (obl_step_dev, storage type).
+   Work memory, allocated by the first call and kept: five spectra of lhx*nyt*(nz+1) complex
+   values, the solve's scratch, and one x-padded field (nxt2*nyt*(nz+1) reals); obl_step_dev
+   takes four of those where they fit in 512 MB together (without that much free memory it
+   runs field by field with one).  An ensemble's instances each hold their own. */
 typedef struct obl_step_io {
     void *u, *v, *w;          /* in/out (ldx,nyt,0:nz), projected in place         */
     const void *theta;        /* in (ldx,nyt,0:nz)                                  */
