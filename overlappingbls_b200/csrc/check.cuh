@@ -19,7 +19,7 @@ namespace obl {
 // check sites (the first failing one is reported)
 enum CheckSite : int {
     CK_COL_LOAD = 1, CK_COL_STORE, CK_ROWS3_ROW, CK_ROWS3_SPEC, CK_TDMA_STORE, CK_TDMA_COPY, CK_PINV_COL_LOAD,
-    CK_PINV_COL_STORE, CK_PINV_ROW, CK_GFORM_LOAD, CK_TDMA_LOAD, CK_SELFTEST
+    CK_PINV_COL_STORE, CK_PINV_ROW, CK_GFORM_LOAD, CK_TDMA_LOAD, CK_SELFTEST, CK_DIVT_ROW
 };
 
 struct CheckRecord {

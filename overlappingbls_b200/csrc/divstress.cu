@@ -26,7 +26,11 @@ __global__ void __launch_bounds__(TpRows<T, N>::NT, TpRows<T, N>::minb)
         return;
     }
     const long long base = (long long)blockIdx.x * WB;
-    auto active = [&](int ln) { return base + ln < a.npairs; };
+    auto active = [&](int ln) {
+        const long long p = base + ln;
+        // checked build: the pair lies in the launch's rows and on one level
+        return p < a.npairs && ck_in(2 * p + 1, 2 * a.npairs, CK_DIVT_ROW) && ck_in((2 * p) % e.ny + 1, e.ny, CK_DIVT_ROW);
+    };
     const long long dz = e.fwd ? e.plane : -e.plane;      // the other tz plane
     {
         constexpr int EL = 128 / sizeof(T), PL = (N + EL - 1) / EL;

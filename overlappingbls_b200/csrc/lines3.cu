@@ -136,6 +136,10 @@ template <int N, int OP> __global__ void __launch_bounds__(32 * kCols3Warps) k_c
     const C *src = reinterpret_cast<const C *>(a.src) + (long long)z * a.src_plane;
     C *dst = reinterpret_cast<C *>(a.dst) + (long long)z * a.dst_plane;
     LineMinor<C, WB> sc{reinterpret_cast<C *>(smraw), line};
+    // the checked build tests each element's level, column and plane offset
+    auto ok = [&](int i, int col, long long row, long long plane, int site) {
+        return ck_in(z, a.nlev, site) && ck_in(col, row, site) && ck_in((long long)i * row + col, plane, site);
+    };
     C v[VR];
 #pragma unroll
     for (int b = 0; b < G0::PER; ++b) {
@@ -145,7 +149,7 @@ template <int N, int OP> __global__ void __launch_bounds__(32 * kCols3Warps) k_c
             const int i = j + r * G0::NB;
             C x = s2(0, 0);
             if (act && (G0::FULL || j < G0::NB)) {
-                x = src[(long long)i * a.src_row + glc];
+                if (!OBL_CHECK || ok(i, glc, a.src_row, a.src_plane, CK_COL_LOAD)) x = src[(long long)i * a.src_row + glc];
                 if (!FWD && kmul) {
                     const float kk = (float)(kmul == 1 ? a.ktab[glc] : a.ktab[i]);
                     x = s2(-kk * x.y, kk * x.x);
@@ -167,7 +171,7 @@ template <int N, int OP> __global__ void __launch_bounds__(32 * kCols3Warps) k_c
                 const int i = j + r * GL::NB;
                 C x = v[b * RL + r];
                 if (FWD && a.zero_nyq && i == N / 2) x = s2(0, 0);
-                dst[(long long)i * a.dst_row + gl] = x;
+                if (!OBL_CHECK || ok(i, gl, a.dst_row, a.dst_plane, CK_COL_STORE)) dst[(long long)i * a.dst_row + gl] = x;
             }
     }
 }
