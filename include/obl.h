@@ -269,9 +269,9 @@ int obl_project_dev(obl_ctx *ctx, void *u, void *v, void *w,
    dpdz and project (103_flosol.f90:168-188).  Pointers are host (obl_step /
    obl_step_f32) or device (obl_step_dev, storage type).
    Work memory, allocated by the first call and kept: five spectra of lhx*nyt*(nz+1) complex
-   values, the solve's scratch, and one x-padded field (nxt2*nyt*(nz+1) reals); obl_step_dev
-   takes four of those where they fit in 512 MB together (without that much free memory it
-   runs field by field with one).  An ensemble's instances each hold their own. */
+   values, the solve's scratch, and one x-padded field (nxt2*nyt*(nz+1) reals).  Where four of
+   those take up to 512 MB together obl_step_dev holds none: the padded outputs big[] carry
+   the x-padded rows on the way.  An ensemble's instances each hold their own. */
 typedef struct obl_step_io {
     void *u, *v, *w;          /* in/out (ldx,nyt,0:nz), projected in place         */
     const void *theta;        /* in (ldx,nyt,0:nz)                                  */

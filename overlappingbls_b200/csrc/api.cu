@@ -68,9 +68,6 @@ struct obl_ctx {
     DevBuf cscr;               // c' scratch
     DevBuf isl_c, isl_d;
     DevBuf tmp;                // pad/unpad intermediate, ifftn temporary
-    DevBuf xpad;               // x-padded fields of the batched forward pass, which leaves tmp
-                               // (and graphs captured with it) alone
-    bool xpad_nomem = false;   // their allocation failed: the pass stays field by field
     DevBuf fscr;               // cluster scratch slots of the fused forward kernel
     // rollout problem of the adjoint: small (ldx,nyt,0:nz) and padded work fields, the
     // per-step state checkpoints and the objective's partial sums
@@ -850,40 +847,33 @@ template <typename T> struct Ops {
     int fwd_lines(const obl_step_io *io)
     {
         int rc;
-        if (fwd_batched()) {
-            // without the memory for four fields' intermediates one field's still does
-            if ((rc = fwd_spec())) return rc;
-            rc = ensure(ctx, ctx->xpad, 4 * xpad_bytes());
-            if (!rc) return fwd_batch(io);
-            if (rc != OBL_ERR_NOMEM) return rc;
-            ctx->xpad_nomem = true;
-            ctx->err.clear();
-        }
+        if (fwd_batched()) return fwd_batch(io);
         if ((rc = fwd_prepare())) return rc;
         for (int c = 0; c < 4; ++c)
             if ((rc = fwd_field(io, c))) return rc;
         return OBL_OK;
     }
-    // All four fields in two launches, rows then columns, instead of fifteen: up to 512 MB of
-    // x-padded intermediates.  Fewer partial last waves, and the column passes of every field
-    // and kind fill one another's gaps.  Step times (us, batched / field by field): 64x64x64
-    // FP64 (13 MB) 71 / 119, 128x128x96 mixed (38 MB) 161 / 218, 256x256x128 (204 MB) 597 /
-    // 692, 512x512x64 (415 MB) 1180 / 1272, 384x384x128 (460 MB) 1308 / 1363; beyond, one
+    // All four fields in two launches, rows then columns, instead of fifteen, where their
+    // x-padded rows are up to 512 MB.  Those wait in the padded outputs themselves, and the
+    // y-pad runs in place: no work buffer, which four fields' rows would fill again for every
+    // context and ensemble instance.  Fewer partial last waves, and the column passes of every
+    // field and kind fill one another's gaps.  Step times (us, batched / field by field):
+    // 64x64x64 FP64 (13 MB) 71 / 119, 128x128x96 mixed (38 MB) 161 / 218, 256x256x128 (204 MB)
+    // 597 / 692, 512x512x64 (415 MB) 1180 / 1272, 384x384x128 (460 MB) 1308 / 1363; beyond, one
     // field's launch fills the GPU and its y-pad has the tensor copies: 512x512x256 (1.6 GB)
     // 4693 / 4630, FP64 10235 / 10001.
     static constexpr size_t kFwdBatchBytes = (size_t)512 << 20;
     size_t xpad_bytes() const { return sizeof(T) * (size_t)ctx->nxt2 * ctx->nyt * (ctx->nz + 1); }
     bool fwd_batched() const
     {
-        return !ctx->param_fwd_chunk && !ctx->xpad_nomem && 4 * xpad_bytes() <= kFwdBatchBytes;
+        return !ctx->param_fwd_chunk && 4 * xpad_bytes() <= kFwdBatchBytes;
     }
     int fwd_batch(const obl_step_io *io)
     {
         const int nlev = ctx->nz + 1, nx = ctx->nxt, ny = ctx->nyt, nx2 = ctx->nxt2, ny2 = ctx->nyt2, lhx = ctx->lhx;
         const long long S = ctx->sp(), pl = ctx->plane(), plx = (long long)nx2 * ny, plb = (long long)nx2 * ny2;
-        const size_t xsz = (size_t)plx * nlev;
         int rc;
-        T *xb = (T *)ctx->xpad.p;
+        if ((rc = fwd_spec())) return rc;
         const T *f[4] = {(const T *)io->u, (const T *)io->v, (const T *)io->w, (const T *)io->theta};
         RowsFwd3Args<T> ra{};
         ra.npairs = (long long)ny * nlev / 2; ra.ldx = ctx->ldx; ra.ny = ny; ra.L = ctx->L; ra.z0 = 0;
@@ -891,16 +881,19 @@ template <typename T> struct Ops {
         ra.kx = ctx->d_kx;
         ra.twF = twt<T>(ctx, nx, ROLE_TP + ROLE_FWD); ra.twB = twt<T>(ctx, nx, ROLE_TP + ROLE_BWD);
         ra.twPB = twt<T>(ctx, nx, ROLE_TP + ROLE_PADBWD);
+        // a plane's x-padded rows are the first ny of its ny2 rows in big: the y-pad's CTAs hold
+        // their columns before they store them
+        ra.xgap = plb - plx;
         RowsFwd3Fields<T> m{};
         ColsFwdArgs<T> ca{};
-        ca.pad = colargs(nullptr, nx2, plx, nullptr, nx2, plb, nx2, nlev, 1.0 / ny, OP_PAD, ny);
+        ca.pad = colargs(nullptr, nx2, plb, nullptr, nx2, plb, nx2, nlev, 1.0 / ny, OP_PAD, ny);
         ca.ddy = colargs(nullptr, ctx->ldx, pl, nullptr, ctx->ldx, pl, nx, nlev, 1.0 / ny, OP_DERIV, ny);
         ca.fwd = colargs(nullptr, lhx, S, nullptr, lhx, S, lhx, ctx->L, 1.0, OP_FWD, ny);
         ca.fwd.zero_nyq = 1;
         ca.nf = 4;
         for (int c = 0; c < 4; ++c) {
             C2<T> *H = c < 3 ? (C2<T> *)ctx->spec[c].p : nullptr;
-            m.src[c] = f[c]; m.dfdx[c] = (T *)io->d[2 * c]; m.xpad[c] = xb + c * xsz; m.H[c] = H;
+            m.src[c] = f[c]; m.dfdx[c] = (T *)io->d[2 * c]; m.xpad[c] = (T *)io->big[c]; m.H[c] = H;
             ca.mpad.src[c] = m.xpad[c]; ca.mpad.dst[c] = io->big[c];
             ca.mddy.src[c] = f[c]; ca.mddy.dst[c] = io->d[2 * c + 1];
             if (H && !(fwd_gform && c != 1)) {   // G form: H_x and H_z are transformed as G in press()
@@ -1706,7 +1699,6 @@ int obl_ctx_destroy(obl_ctx *ctx)
     cudaFree(ctx->isl_c.p);
     cudaFree(ctx->isl_d.p);
     cudaFree(ctx->tmp.p);
-    cudaFree(ctx->xpad.p);
     cudaFree(ctx->fscr.p);
     for (auto &b : ctx->rw_small) cudaFree(b.p);
     for (auto &b : ctx->rw_big) cudaFree(b.p);

@@ -259,9 +259,10 @@ __global__ void __launch_bounds__(256, 2) k_fwd_fused(FwdFusedArgs<T> a)
 template <typename T> struct RowsFwd3Args {
     const T *src;          // field (ldx, ny, nlev)
     T *dfdx;               // (ldx, ny, nlev)
-    T *xpad;               // (nx2, ny, nlev)
+    T *xpad;               // (nx2, ny, nlev), xgap more elements between the levels
     C2<T> *H;              // (lhx, ny, nlev) or nullptr (theta)
     long long npairs;      // ny*nlev/2
+    long long xgap;
     int ldx, ny, L;
     int z0;                // level of the first row pair (src, dfdx, H start there; a chunk of levels)
     double sc_press;
@@ -359,7 +360,7 @@ __device__ __forceinline__ void tp_rows_fwd3_unit(const RowsFwd3Args<T> &a, long
             if (!active(ln)) return;
             const long long r0 = 2 * (base + ln);
             const T ca = a.src[r0 * a.ldx], cb = a.src[(r0 + 1) * a.ldx];
-            T *A = a.xpad + r0 * N2, *B = A + N2;
+            T *A = a.xpad + (a.xgap ? r0 * N2 + (r0 / a.ny) * a.xgap : r0 * N2), *B = A + N2;
 #pragma unroll
             for (int r = 0; r < R0; ++r) {
                 A[jj + r * RP] = x[r].x + ca;

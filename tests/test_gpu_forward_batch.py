@@ -123,21 +123,21 @@ def test_batched_step_under_index_checks():
     assert r.returncode == 0 and "28 passed" in tail, tail
 
 
-def test_step_without_memory_for_the_batch(orc):
-    """The sixth allocation of a first device step (after the five spectra) is the batch's
-    intermediates; without it the step runs field by field, with one field's."""
-    ctx, g, f = _setup(orc, 64, 48, 17, "f64")
+def test_batch_holds_no_buffer_of_its_own(orc):
+    """The x-padded rows wait in the padded outputs: a first device step allocates the five
+    spectra and the solve's c', and no seventh buffer."""
+    ctx, g, f = _setup(orc, 64, 48, 10, "f64")
     s = DevStep(ctx, f, "f64")
-    ctx.set_param("fail_alloc", 6)
-    names = _launches(ctx, s.run)
-    assert ctx.get_param("fail_alloc") == 0 and "pad_cols" in names and "cols_fwd" not in names, names
-    s.check(g.step(f["u"], f["v"], f["w"], f["theta"], npz=2), TOL["f64"])
+    ctx.set_param("fail_alloc", 7)     # spectra 5, c' 1
+    s.run()
+    assert ctx.get_param("fail_alloc") == 1
+    s.check(g.step(f["u"], f["v"], f["w"], f["theta"], npz=3), TOL["f64"])
     ctx.close()
 
 
 def test_captured_call_survives_a_first_step(orc):
-    """A step's memory is its own: the intermediate of a zero_padding captured in a CUDA
-    graph stays where it was when the context then makes its first step."""
+    """The intermediate of a zero_padding captured in a CUDA graph stays where it was when
+    the context then makes its first step."""
     import torch
     ctx, g, f = _setup(orc, 64, 48, 17, "f64")
     s = DevStep(ctx, f, "f64")
